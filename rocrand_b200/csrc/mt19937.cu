@@ -17,11 +17,12 @@
 //
 // Seeding (mt19937.hpp:83-206): generator e starts from the Knuth state of
 // (seed >> 32) ^ seed advanced by e * 2^1000 steps.  A jump polynomial p applied to a state
-// whose continuation is x gives word k = XOR of x[i + k] over the set coefficients i of p,
-// so each block extends its start state to 20560 words in shared memory and lets 624
-// threads accumulate one word each.  The polynomials (x^(i 2^1000) and x^(256 i 2^1000)
-// mod the characteristic polynomial) are derived at build time by
-// rocrand_b200/data/make_mt19937_jump.c and embedded by mt19937_data.S.
+// whose continuation is x gives word k = XOR of x[i + k] over the set coefficients i of p.
+// With e = e0 + 256 e1 the seed state is first moved by e1 * 256 * 2^1000 (31 polynomials),
+// then each of the 32 states by e0 * 2^1000 (255 polynomials, eight coefficients at a time:
+// mt_jump_low).  The polynomials (x^(i 2^1000) and x^(256 i 2^1000) mod the characteristic
+// polynomial) are derived at build time by rocrand_b200/data/make_mt19937_jump.c and embedded
+// by mt19937_data.S.
 #include "common.hpp"
 #include "dist.cuh"
 #include "generators.hpp"
@@ -51,7 +52,19 @@ constexpr unsigned kMtSlots   = 78;
 constexpr unsigned kMtSeq     = 19937 + kMtN - 1; // a state and the 19936 words after it
 constexpr unsigned kMtPolys   = 255 + 31;
 constexpr unsigned kMtBlock   = 64;
-constexpr unsigned kJumpBlock = 640;
+// seeding
+constexpr unsigned kMtHigh     = 32;    // start states: second digit of e
+constexpr unsigned kMtSeqPad   = 20640; // a stored sequence: kMtSeq words, then zeros to the last column read
+constexpr unsigned kSeqBlock   = 256;
+constexpr unsigned kJumpBlock  = 640;
+constexpr unsigned kHighSplit  = 16;               // blocks per polynomial of mt_jump_high
+constexpr unsigned kLowLanes   = 40;               // threads across a slice, four words each
+constexpr unsigned kLowCols    = 4 * kLowLanes;    // words per slice: four slices cover 624
+constexpr unsigned kLowThreads = 16 * kLowLanes;   // 16 groups of 16 generators
+constexpr unsigned kRingChunks = 7;                // window: six chunks in use, one being made
+constexpr unsigned kRowBytes   = 128 * kRingChunks;
+static_assert(kMtN % kHighSplit == 0, "whole coefficient words per block");
+static_assert(3 * kLowCols + 32 * (kMtN + 4) + 31 + 7 < kMtSeqPad, "the last new column lies in the padding");
 constexpr uint32_t kFullMask  = 0xffffffffu;
 
 __host__ __device__ __forceinline__ uint32_t mt_mix(uint32_t a, uint32_t b, uint32_t m)
@@ -161,27 +174,15 @@ __device__ __forceinline__ void word_home(unsigned k, unsigned& lane, unsigned& 
     slot             = 1 + 7 * i + d % 7;
 }
 
-// XOR of x[i + k] over the set coefficients i of `poly` (all threads read the same bits).
-__device__ __forceinline__ uint32_t apply_poly(const uint32_t* poly, const uint32_t* x, unsigned k)
+// The seed state travels as a kernel parameter.
+struct MtSeed
 {
-    uint32_t acc = 0;
-    for(unsigned w = 0; w < kMtN; w++)
-    {
-        uint32_t        bits = poly[w];
-        const uint32_t* base = x + 32 * w + k;
-        while(bits)
-        {
-            const int b = __ffs(bits) - 1;
-            bits &= bits - 1;
-            acc ^= base[b];
-        }
-    }
-    return acc;
-}
+    uint32_t w[kMtN];
+};
 
-// Extends the state sh[0..623] to kMtSeq words in place (227 words per step: word k reads
-// k-624, k-623 and k-227).
-__device__ __forceinline__ void extend_sequence(uint32_t* sh)
+// Continues a state to kMtSeqPad words at `out` (227 words per step: word k reads k-624,
+// k-623 and k-227); the words after kMtSeq are zero (no polynomial reaches them).
+__device__ __forceinline__ void write_sequence(uint32_t* sh, uint32_t* __restrict__ out)
 {
     for(unsigned c = kMtN; c < kMtSeq; c += kMtN - kMtM)
     {
@@ -190,62 +191,185 @@ __device__ __forceinline__ void extend_sequence(uint32_t* sh)
             sh[k] = mt_mix(sh[k - kMtN], sh[k - kMtN + 1], sh[k - (kMtN - kMtM)]);
         __syncthreads();
     }
+    for(unsigned k = threadIdx.x; k < kMtSeqPad; k += blockDim.x)
+        out[k] = k < kMtSeq ? sh[k] : 0u;
 }
 
-// Block e0 = 1..255: the seed state advanced by e0 * 2^1000 (first radix-256 digit).
-__global__ __launch_bounds__(kJumpBlock) void mt_jump_low(const uint32_t* __restrict__ seed_state,
-                                                         const uint32_t* __restrict__ polys,
-                                                         uint32_t* __restrict__ low_states)
+// Sequence 0: the seed state's continuation.  The 31 other start states are cleared for
+// mt_jump_high, which XORs into them.
+__global__ __launch_bounds__(kSeqBlock) void mt_seed_sequence(const __grid_constant__ MtSeed seed,
+                                                             uint32_t* __restrict__ starts,
+                                                             uint32_t* __restrict__ seqs)
 {
     extern __shared__ uint32_t sh[];
-    uint32_t*      poly = sh + kMtSeq;
-    const unsigned e0   = blockIdx.x + 1;
     for(unsigned k = threadIdx.x; k < kMtN; k += blockDim.x)
-    {
-        sh[k]   = seed_state[k];
-        poly[k] = polys[(e0 - 1) * kMtN + k];
-    }
+        sh[k] = seed.w[k];
+    for(unsigned k = threadIdx.x; k < kMtHigh * kMtN; k += blockDim.x)
+        starts[k] = 0u;
     __syncthreads();
-    extend_sequence(sh);
-    if(threadIdx.x < kMtN)
-        low_states[e0 * kMtN + threadIdx.x] = apply_poly(poly, sh, threadIdx.x);
+    write_sequence(sh, seqs);
 }
 
-// Block e = 0..8191: generator e's start state (second digit e / 256 applied to the
-// first-digit state of e % 256), scattered into the lane/slot arena.
-__global__ __launch_bounds__(kJumpBlock) void mt_jump_high(const uint32_t* __restrict__ seed_state,
-                                                          const uint32_t* __restrict__ low_states,
-                                                          const uint32_t* __restrict__ polys,
-                                                          uint32_t* __restrict__ arena)
+// Sequences 1..31 from their start states.
+__global__ __launch_bounds__(kSeqBlock) void mt_sequences(const uint32_t* __restrict__ starts,
+                                                         uint32_t* __restrict__ seqs)
 {
     extern __shared__ uint32_t sh[];
-    uint32_t*       poly = sh + kMtSeq;
-    const unsigned  e    = blockIdx.x;
-    const unsigned  e0 = e % 256, e1 = e / 256;
-    const uint32_t* src  = e0 == 0 ? seed_state : low_states + e0 * kMtN;
+    const unsigned e1 = blockIdx.x + 1;
     for(unsigned k = threadIdx.x; k < kMtN; k += blockDim.x)
+        sh[k] = starts[e1 * kMtN + k];
+    __syncthreads();
+    write_sequence(sh, seqs + static_cast<size_t>(e1) * kMtSeqPad);
+}
+
+// Start state e1 = 1..31 (blockIdx.x + 1): polynomial e1 * 256 * 2^1000 applied to the seed's
+// sequence.  The 624 coefficient words are split over kHighSplit blocks, whose partial sums
+// meet by atomic XOR: one block per polynomial would be a chain of 10000 additions.
+__global__ __launch_bounds__(kJumpBlock) void mt_jump_high(const uint32_t* __restrict__ polys,
+                                                          const uint32_t* __restrict__ seqs,
+                                                          uint32_t* __restrict__ starts)
+{
+    constexpr unsigned  kWords = kMtN / kHighSplit;
+    __shared__ uint32_t x[32 * kWords + kMtN];
+    const unsigned      e1 = blockIdx.x + 1;
+    const unsigned      w0 = blockIdx.y * kWords;
+    for(unsigned k = threadIdx.x; k < 32 * kWords + kMtN; k += blockDim.x)
+        x[k] = seqs[32 * w0 + k];
+    __syncthreads();
+    if(threadIdx.x >= kMtN)
+        return;
+    const uint32_t* poly = polys + (255 + e1 - 1) * kMtN + w0;
+    uint32_t        acc  = 0;
+    for(unsigned w = 0; w < kWords; w++)
     {
-        sh[k] = src[k];
-        if(e1 != 0)
-            poly[k] = polys[(255 + e1 - 1) * kMtN + k];
+        uint32_t        bits = poly[w];
+        const uint32_t* base = x + 32 * w + threadIdx.x;
+        while(bits)
+        {
+            const int b = __ffs(bits) - 1;
+            bits &= bits - 1;
+            acc ^= base[b];
+        }
+    }
+    atomicXor(starts + e1 * kMtN + threadIdx.x, acc);
+}
+
+// Rows v = 16 wq .. 16 wq + 15 of the subset sums of eight consecutive sequence words (lane's
+// column n): row v, column n = XOR of x[n + b] over the set bits b of v.
+__device__ __forceinline__ void write_subset_rows(unsigned char* col, unsigned wq, const uint32_t (&x)[8])
+{
+    uint32_t hi = (wq & 1u ? x[4] : 0u) ^ (wq & 2u ? x[5] : 0u) ^ (wq & 4u ? x[6] : 0u) ^ (wq & 8u ? x[7] : 0u);
+    unsigned char* p = col + wq * 16u * kRowBytes;
+#pragma unroll
+    for(unsigned v = 0; v < 16; v++)
+    {
+        uint32_t lo = hi;
+#pragma unroll
+        for(unsigned b = 0; b < 4; b++)
+            if((v >> b) & 1u)
+                lo ^= x[b];
+        *reinterpret_cast<uint32_t*>(p + v * kRowBytes) = lo;
+    }
+}
+
+__device__ __forceinline__ uint4 xor3(uint4 a, uint4 b, uint4 c)
+{
+    return make_uint4(a.x ^ b.x ^ c.x, a.y ^ b.y ^ c.y, a.z ^ b.z ^ c.z, a.w ^ b.w ^ c.w);
+}
+
+// All 8192 start states: block (slice, e1) computes words 160 slice .. of the generators
+// e = e0 + 256 e1, e0 < 256.  Eight coefficients i = 8g .. 8g+7 of polynomial e0 select one of
+// 256 subset sums of x[8g + k .. 8g + k + 7]; since that sum depends on 8g + k only, row v of
+// the table is one long array that every group reads at its own offset, so a sliding window
+// of it is kept in shared memory (seven chunks of 32 columns x 256 rows, 224 KB) and each
+// sum is made once: 32 new columns per 32 coefficients.  A thread keeps 16 generators x 4
+// words; a group costs it 16 16-byte reads (conflict-free: eight lanes read 128 contiguous
+// bytes of one row), which bound the kernel: 128 blocks x 624 chunks x 5120 shared-memory
+// wavefronts = 1.63 ms at 1965 MHz.
+// The coefficient-at-a-time form this replaces took 23.4 ms (one 4-byte read per set
+// coefficient, word and generator); a whole set_seed + 2^20 uniforms went from 24.30 ms to
+// 2.47 ms.
+__global__ __launch_bounds__(kLowThreads, 1) void mt_jump_low(const uint32_t* __restrict__ seqs,
+                                                             const uint4* __restrict__ coeffs,
+                                                             uint32_t* __restrict__ arena)
+{
+    extern __shared__ __align__(128) unsigned char tab[];
+    const unsigned  tid   = threadIdx.x;
+    const unsigned  group = tid / kLowLanes, col = tid % kLowLanes;
+    const unsigned  warp = tid >> 5, lane = tid & 31u;
+    const unsigned  k0 = blockIdx.x * kLowCols, e1 = blockIdx.y;
+    const uint32_t* x    = seqs + static_cast<size_t>(e1) * kMtSeqPad + k0 + lane;
+    uint4           acc[16];
+#pragma unroll
+    for(int i = 0; i < 16; i++)
+        acc[i] = make_uint4(0u, 0u, 0u, 0u);
+
+    // window: chunk c (columns 32c .. 32c+31) lives in ring slot c % 7; a chunk's four groups
+    // read columns of chunks c .. c+5
+    if(warp < 16)
+    {
+        for(unsigned c = 0; c < kRingChunks - 1; c++)
+        {
+            uint32_t xs[8];
+#pragma unroll
+            for(int b = 0; b < 8; b++)
+                xs[b] = x[32 * c + b];
+            write_subset_rows(tab + (32 * c + lane) * 4, warp, xs);
+        }
     }
     __syncthreads();
-    uint32_t word = 0;
-    if(e1 != 0)
+
+    unsigned pos  = 16u * col;                      // byte offset in a row of this thread's columns
+    unsigned fill = 128u * (kRingChunks - 1);       // byte offset in a row of the next new chunk
+    const uint4* cf = coeffs + group;               // 16 generators' bytes of one group
+    for(unsigned q = 0; q < kMtN; q++)
     {
-        extend_sequence(sh);
-        if(threadIdx.x < kMtN)
-            word = apply_poly(poly, sh, threadIdx.x);
+#pragma unroll 1
+        for(unsigned h = 0; h < 2; h++)
+        {
+            const uint4          ca = __ldg(cf), cb = __ldg(cf + 16);
+            const unsigned       pa = pos, pb = pos + 32u < kRowBytes ? pos + 32u : pos + 32u - kRowBytes;
+            const uint32_t       wa[4] = {ca.x, ca.y, ca.z, ca.w}, wb[4] = {cb.x, cb.y, cb.z, cb.w};
+            cf += 32;
+            pos = pb + 32u < kRowBytes ? pb + 32u : pb + 32u - kRowBytes;
+#pragma unroll
+            for(unsigned i = 0; i < 16; i++)
+            {
+                const uint32_t va = __byte_perm(wa[i / 4], 0u, 0x4440u | (i % 4));
+                const uint32_t vb = __byte_perm(wb[i / 4], 0u, 0x4440u | (i % 4));
+                acc[i] = xor3(acc[i], *reinterpret_cast<const uint4*>(tab + (va * kRowBytes + pa)),
+                              *reinterpret_cast<const uint4*>(tab + (vb * kRowBytes + pb)));
+            }
+            // the next chunk, between the two halves: the warps that wait for its words leave the
+            // shared-memory pipe to the others
+            if(h == 0 && warp < 16 && q + kRingChunks - 1 <= kMtN + 4)
+            {
+                uint32_t xs[8];
+#pragma unroll
+                for(int b = 0; b < 8; b++)
+                    xs[b] = x[32 * (q + kRingChunks - 1) + b];
+                write_subset_rows(tab + fill + 4 * lane, warp, xs);
+            }
+        }
+        fill = fill + 128u < kRowBytes ? fill + 128u : 0u;
+        __syncthreads();
     }
-    else if(threadIdx.x < kMtN)
+
+    const unsigned k = k0 + 4 * col;
+    if(k >= kMtN) // 624 is a multiple of 4: a thread's words are all in or all out
+        return;
+#pragma unroll
+    for(unsigned j = 0; j < 4; j++)
     {
-        word = sh[threadIdx.x];
-    }
-    if(threadIdx.x < kMtN)
-    {
-        unsigned lane, slot;
-        word_home(threadIdx.x, lane, slot);
-        arena[slot * kMtThreads + e * 8 + lane] = word;
+        unsigned mt_lane = 0, slot = 0;
+        word_home(k + j, mt_lane, slot);
+        uint32_t* out = arena + static_cast<size_t>(slot) * kMtThreads + (group * 16u + 256u * e1) * 8u + mt_lane;
+#pragma unroll
+        for(unsigned i = 0; i < 16; i++)
+        {
+            const uint32_t w[4] = {acc[i].x, acc[i].y, acc[i].z, acc[i].w};
+            out[i * 8u] = w[j];
+        }
     }
 }
 
@@ -526,7 +650,12 @@ __global__ __launch_bounds__(kMtBlock, 7) void mt_fill(MtArgs a, F fw)
     }
 }
 
-// Jump polynomials on each device, uploaded once.
+// Jump polynomials on each device, uploaded once: the 286 polynomials as derived (mt_jump_high
+// reads the last 31), then the first digit's coefficients by group of eight -- byte e0 of
+// row g holds coefficients 8g .. 8g+7 of x^(e0 2^1000) (e0 = 0: the polynomial 1).
+constexpr size_t kMtPolyWords  = static_cast<size_t>(kMtPolys) * kMtN;
+constexpr size_t kMtCoeffBytes = static_cast<size_t>(4 * kMtN) * 256;
+
 const uint32_t* device_jump_polys()
 {
     static std::mutex                   mu;
@@ -536,13 +665,20 @@ const uint32_t* device_jump_polys()
     if(ptr[dev])
         return ptr[dev];
     const size_t words = static_cast<size_t>(rb200_mt19937_jump_end - rb200_mt19937_jump_begin);
-    if(words != static_cast<size_t>(kMtPolys) * kMtN)
+    if(words != kMtPolyWords)
         return nullptr;
+    std::vector<unsigned char> host(words * sizeof(uint32_t) + kMtCoeffBytes);
+    std::memcpy(host.data(), rb200_mt19937_jump_begin, words * sizeof(uint32_t));
+    unsigned char* coeff = host.data() + words * sizeof(uint32_t);
+    coeff[0]             = 1;
+    for(unsigned e0 = 1; e0 < 256; e0++)
+        for(unsigned g = 0; g < 4 * kMtN; g++)
+            coeff[static_cast<size_t>(g) * 256 + e0] = static_cast<unsigned char>(
+                rb200_mt19937_jump_begin[static_cast<size_t>(e0 - 1) * kMtN + g / 4] >> (8 * (g % 4)));
     void* d = nullptr;
-    if(cudaMalloc(&d, words * sizeof(uint32_t)) != cudaSuccess)
+    if(cudaMalloc(&d, host.size()) != cudaSuccess)
         return nullptr;
-    if(cudaMemcpy(d, rb200_mt19937_jump_begin, words * sizeof(uint32_t), cudaMemcpyHostToDevice)
-       != cudaSuccess)
+    if(cudaMemcpy(d, host.data(), host.size(), cudaMemcpyHostToDevice) != cudaSuccess)
     {
         cudaFree(d);
         return nullptr;
@@ -571,7 +707,7 @@ inline void mt_twist_host(uint32_t* s)
         s[i] = mt_mix(s[i], s[(i + 1) % kMtN], s[(i + kMtM) % kMtN]);
 }
 
-// x[0..623] extended to kMtSeq words (the host form of extend_sequence).
+// x[0..623] extended to kMtSeq words (the host form of write_sequence).
 inline void mt_sequence_host(const uint32_t* state, uint32_t* x)
 {
     std::memcpy(x, state, sizeof(uint32_t) * kMtN);
@@ -757,41 +893,40 @@ public:
         const uint32_t* polys = device_jump_polys();
         if(polys == nullptr)
             return ROCRAND_STATUS_ALLOCATION_FAILED;
+        // the state arena, then the seeding scratch: 32 start states and their sequences
         constexpr size_t kArenaWords = static_cast<size_t>(kMtSlots) * kMtThreads;
-        constexpr size_t kLowWords   = 256 * kMtN;
+        constexpr size_t kStartWords = static_cast<size_t>(kMtHigh) * kMtN;
+        constexpr size_t kSeqWords   = static_cast<size_t>(kMtHigh) * kMtSeqPad;
         if(m_arena == nullptr)
         {
-            if(cudaMalloc(&m_arena, sizeof(uint32_t) * (kArenaWords + kLowWords + kMtN))
+            if(cudaMalloc(&m_arena, sizeof(uint32_t) * (kArenaWords + kStartWords + kSeqWords))
                != cudaSuccess)
             {
                 m_arena = nullptr;
                 return ROCRAND_STATUS_ALLOCATION_FAILED;
             }
         }
-        uint32_t* low  = m_arena + kArenaWords;
-        uint32_t* seed = low + kLowWords;
+        uint32_t* starts = m_arena + kArenaWords;
+        uint32_t* seqs   = starts + kStartWords;
         // Knuth initialisation of (seed >> 32) ^ seed (mt19937.hpp:107-116)
-        uint32_t s[kMtN];
-        s[0] = static_cast<uint32_t>((m_seed >> 32) ^ m_seed);
+        MtSeed s;
+        s.w[0] = static_cast<uint32_t>((m_seed >> 32) ^ m_seed);
         for(uint32_t i = 1; i < kMtN; i++)
-            s[i] = 1812433253u * (s[i - 1] ^ (s[i - 1] >> 30)) + i;
-        // pageable source: the copy has read it when cudaMemcpyAsync returns
-        if(cudaMemcpyAsync(seed, s, sizeof(s), cudaMemcpyHostToDevice, m_stream) != cudaSuccess)
-            return ROCRAND_STATUS_INTERNAL_ERROR;
-        const size_t smem = sizeof(uint32_t) * (kMtSeq + kMtN);
-        if(cudaFuncSetAttribute(mt_jump_low, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(smem))
-               != cudaSuccess
-           || cudaFuncSetAttribute(mt_jump_high, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(smem))
-                  != cudaSuccess)
+            s.w[i] = 1812433253u * (s.w[i - 1] ^ (s.w[i - 1] >> 30)) + i;
+        const size_t seq_smem = sizeof(uint32_t) * kMtSeq;
+        const size_t low_smem = 256 * kRowBytes;
+        auto         allow    = [](auto k, size_t bytes) {
+            return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes))
+                   == cudaSuccess;
+        };
+        if(!allow(mt_seed_sequence, seq_smem) || !allow(mt_sequences, seq_smem) || !allow(mt_jump_low, low_smem))
             return ROCRAND_STATUS_LAUNCH_FAILURE;
-        mt_jump_low<<<255, kJumpBlock, smem, m_stream>>>(seed, polys, low);
-        rocrand_status st = launch_status();
-        if(st != ROCRAND_STATUS_SUCCESS)
-            return st;
-        mt_jump_high<<<kMtGens, kJumpBlock, smem, m_stream>>>(seed, low, polys, m_arena);
-        st = launch_status();
+        mt_seed_sequence<<<1, kSeqBlock, seq_smem, m_stream>>>(s, starts, seqs);
+        mt_jump_high<<<dim3(kMtHigh - 1, kHighSplit), kJumpBlock, 0, m_stream>>>(polys, seqs, starts);
+        mt_sequences<<<kMtHigh - 1, kSeqBlock, seq_smem, m_stream>>>(starts, seqs);
+        mt_jump_low<<<dim3((kMtN + kLowCols - 1) / kLowCols, kMtHigh), kLowThreads, low_smem, m_stream>>>(
+            seqs, reinterpret_cast<const uint4*>(polys + kMtPolyWords), m_arena);
+        const rocrand_status st = launch_status();
         if(st != ROCRAND_STATUS_SUCCESS)
             return st;
         m_start       = 0;
