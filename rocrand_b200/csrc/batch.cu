@@ -239,6 +239,24 @@ __device__ __forceinline__ void stateful_tile(const BatchReq& r, unsigned long l
         uint32_t           in[F::iw];
         T                  out[F::ow];
         unsigned long long j = t;
+        if constexpr(has_pair<F>::value)
+        {
+            // two vectors' units side by side
+            for(; j + kBatchE < r.vec_n; j += 2 * kBatchE)
+            {
+                uint32_t in1[F::iw];
+                T        out1[F::ow];
+#pragma unroll
+                for(unsigned i = 0; i < F::iw; i++)
+                    in[i] = eng.next();
+#pragma unroll
+                for(unsigned i = 0; i < F::iw; i++)
+                    in1[i] = eng.next();
+                f.pair(in, in1, out, out1);
+                store_small(r.vec + j * VB, out);
+                store_small(r.vec + (j + kBatchE) * VB, out1);
+            }
+        }
         for(; j < r.vec_n; j += kBatchE)
         {
 #pragma unroll

@@ -6,8 +6,9 @@
 // against the reference's host generators.  Every rounding step is written with an
 // explicit _rn intrinsic: a product is fused into an FMA only where it is exact (scaling
 // by a power of two), so the device rounds exactly where the x86-64 host does.
-// fp32 transcendentals use CUDA's accurate library functions, within an ulp or two of the
-// host C library, inside the stated fp32 tolerance.  The fp64 Box-Muller transforms and
+// The fp32 and half Box-Muller transforms run on two units at a time (normal_math.cuh) on the
+// device, within an ulp or two of the host C library, inside the stated fp32 tolerance; the
+// log-normals' exponential is CUDA's.  The fp64 Box-Muller transforms and
 // the inverse-erf normal take log/sin/cos from precise_math.cuh (correctly rounded but for
 // rare near-halfway cases), so that the fp64 outputs stay within 2 ulp of the host's and
 // the ill-conditioned inverse-erf formula starts from the same logarithm wherever the host
@@ -17,6 +18,7 @@
 #include <type_traits>
 #include "common.hpp"
 #include "ieee.cuh"
+#include "normal_math.cuh"
 #include "precise_math.cuh"
 
 #include <cuda_fp16.h>
@@ -64,15 +66,163 @@ RB_HD __half u16_to_f16(uint32_t v16)
     return __float2half_rn(ieee::ffma((float)(v16 & 0xffffu), RB_2POW16_INV, RB_2POW16_INV));
 }
 
-// rocrand_normal.h:51-66 (host branch: sinf/cosf on the rounded angle).
-RB_HD float2 box_muller_f32(uint32_t x, uint32_t y)
+// The Box-Muller products of a unit on the host: (sin a, cos a) sqrt(-2 log u) with the C
+// library's functions, every step rounded (rocrand_normal.h:51-66, host branch).
+inline float2 box_muller_host(float u, float a)
 {
-    const float u = ieee::ffma(ieee::u2f(x), RB_2POW32_INV, RB_2POW32_INV);
-    const float v = ieee::fadd(RB_2POW32_INV_2PI, ieee::fmul(ieee::u2f(y), RB_2POW32_INV_2PI));
-    const float s = ieee::fsqrt(ieee::fmul(-2.0f, ieee::logf_(u)));
-    float       sv, cv;
-    ieee::sincosf_(v, &sv, &cv);
-    return make_float2(ieee::fmul(sv, s), ieee::fmul(cv, s));
+    const float s = ieee::fsqrt(ieee::fmul(-2.0f, std::log(u)));
+    return make_float2(ieee::fmul(std::sin(a), s), ieee::fmul(std::cos(a), s));
+}
+
+// ---- fp32 and half Box-Muller functors: two units at a time ----
+// Such a functor names the uniforms and angles of two units (`uniforms`, `angles`: the inputs'
+// own rounding steps) and its parameters; normal_pair makes both units' outputs.  On the device one unit alone is the same computation with the unit taken twice, so
+// a value does not depend on whether it was made alone or beside another; on the host each
+// unit is made with the C library.
+
+// rocrand_uniform.h:61-64 and rocrand_normal.h:51-66 of two 32-bit words.
+RB_HD nm::F2 uniform_pair(uint32_t x0, uint32_t x1)
+{
+    return nm::fma(nm::pack(ieee::u2f(x0), ieee::u2f(x1)), nm::rep(RB_2POW32_INV), nm::rep(RB_2POW32_INV));
+}
+// (The products are scalar: packed ones are fused with the packed sum, which rounds once where
+// the reference rounds twice.)
+RB_HD nm::F2 angle_pair(uint32_t y0, uint32_t y1)
+{
+    return nm::add(nm::pack(ieee::fmul(ieee::u2f(y0), RB_2POW32_INV_2PI), ieee::fmul(ieee::u2f(y1), RB_2POW32_INV_2PI)),
+                   nm::rep(RB_2POW32_INV_2PI));
+}
+
+template<class F, class W>
+inline float2 box_muller_host(const F& f, const W* in)
+{
+    float u, a, unused;
+    nm::unpack(f.uniforms(in, in), u, unused);
+    nm::unpack(f.angles(in, in), a, unused);
+    return box_muller_host(u, a);
+}
+
+template<class F>
+RB_HD void exponentials(const F& f, float (&out)[2])
+{
+    if(f.exponential())
+    {
+        out[0] = ieee::expf_(out[0]);
+        out[1] = ieee::expf_(out[1]);
+    }
+}
+
+// The half outputs of one unit from its products (rocrand_normal.h:102-122, float branch used by
+// the host build: halves of the products first).
+template<class F>
+RB_HD void finish_f16(const F& f, float s, float c, __half* out)
+{
+    const float z = ieee::fadd(f.mean, ieee::fmul(f.stddev, __half2float(__float2half_rn(s))));
+    const float w = ieee::fadd(f.mean, ieee::fmul(f.stddev, __half2float(__float2half_rn(c))));
+    out[0]        = __float2half_rn(f.exponential() ? ieee::expf_(z) : z);
+    out[1]        = __float2half_rn(f.exponential() ? ieee::expf_(w) : w);
+}
+
+template<class F, class W>
+RB_HD void normal_pair(const F& f, const W* in0, const W* in1, float* out0, float* out1)
+{
+    float a[2], b[2];
+#if defined(__CUDA_ARCH__)
+    nm::F2 ps, pc;
+    nm::box_muller(f.uniforms(in0, in1), f.angles(in0, in1), ps, pc);
+    const nm::F2 m = nm::rep(f.mean), d = nm::rep(f.stddev);
+    nm::unpack(nm::fma(ps, d, m), a[0], b[0]);
+    nm::unpack(nm::fma(pc, d, m), a[1], b[1]);
+#else
+    const float2 v = box_muller_host(f, in0), w = box_muller_host(f, in1);
+    a[0] = ieee::fadd(f.mean, ieee::fmul(v.x, f.stddev));
+    a[1] = ieee::fadd(f.mean, ieee::fmul(v.y, f.stddev));
+    b[0] = ieee::fadd(f.mean, ieee::fmul(w.x, f.stddev));
+    b[1] = ieee::fadd(f.mean, ieee::fmul(w.y, f.stddev));
+#endif
+    exponentials(f, a);
+    exponentials(f, b);
+    out0[0] = a[0];
+    out0[1] = a[1];
+    out1[0] = b[0];
+    out1[1] = b[1];
+}
+
+template<class F, class W>
+RB_HD void normal_pair(const F& f, const W* in0, const W* in1, __half* out0, __half* out1)
+{
+#if defined(__CUDA_ARCH__)
+    nm::F2 ps, pc;
+    float  s0, s1, c0, c1;
+    nm::box_muller(f.uniforms(in0, in1), f.angles(in0, in1), ps, pc);
+    nm::unpack(ps, s0, s1);
+    nm::unpack(pc, c0, c1);
+    finish_f16(f, s0, c0, out0);
+    finish_f16(f, s1, c1, out1);
+#else
+    const float2 v = box_muller_host(f, in0), w = box_muller_host(f, in1);
+    finish_f16(f, v.x, v.y, out0);
+    finish_f16(f, w.x, w.y, out1);
+#endif
+}
+
+// One unit alone.
+template<class F, class W, class T>
+RB_HD void normal_unit(const F& f, const W* in, T* out)
+{
+#if defined(__CUDA_ARCH__)
+    T unused[2];
+    normal_pair(f, in, in, out, unused);
+#else
+    const float2 v = box_muller_host(f, in);
+    if constexpr(std::is_same_v<T, float>)
+    {
+        float a[2] = {ieee::fadd(f.mean, ieee::fmul(v.x, f.stddev)), ieee::fadd(f.mean, ieee::fmul(v.y, f.stddev))};
+        exponentials(f, a);
+        out[0] = a[0];
+        out[1] = a[1];
+    }
+    else
+    {
+        finish_f16(f, v.x, v.y, out);
+    }
+#endif
+}
+
+RB_HD nm::F2 uniform_pair_f16(uint32_t x0, uint32_t x1)
+{
+    return nm::fma(nm::pack(static_cast<float>(x0), static_cast<float>(x1)), nm::rep(RB_2POW16_INV),
+                   nm::rep(RB_2POW16_INV));
+}
+RB_HD nm::F2 angle_pair_f16(uint32_t y0, uint32_t y1)
+{
+    return nm::add(nm::pack(ieee::fmul(static_cast<float>(y0), RB_2POW16_INV_2PI),
+                            ieee::fmul(static_cast<float>(y1), RB_2POW16_INV_2PI)),
+                   nm::rep(RB_2POW16_INV_2PI));
+}
+
+// Two units of any functor: side by side where it has a form for that, one after the other
+// elsewhere.
+template<class F, class = void>
+struct has_pair : std::false_type
+{
+};
+template<class F>
+struct has_pair<F, std::enable_if_t<F::kPair>> : std::true_type
+{
+};
+template<class F, class W>
+RB_HD void apply_pair(const F& f, const W* in0, const W* in1, typename F::T* out0, typename F::T* out1)
+{
+    if constexpr(has_pair<F>::value)
+    {
+        f.pair(in0, in1, out0, out1);
+    }
+    else
+    {
+        f(in0, out0);
+        f(in1, out1);
+    }
 }
 
 // rocrand_normal.h:68-89 (host branch: sin/cos of w * pi rounded in double).
@@ -87,18 +237,6 @@ RB_HD double2 box_muller_f64(uint32_t x, uint32_t y, uint32_t z, uint32_t w)
     double         sv, cv;
     pm::sincos(a, sv, cv);
     return make_double2(ieee::dmul(sv, s), ieee::dmul(cv, s));
-}
-
-// rocrand_normal.h:102-122, float branch used by the host build; halves of the results.
-RB_HD void box_muller_f16(uint32_t v, __half r[2])
-{
-    const float u = ieee::ffma((float)(v & 0xffffu), RB_2POW16_INV, RB_2POW16_INV);
-    const float a = ieee::fadd(RB_2POW16_INV_2PI, ieee::fmul((float)(v >> 16), RB_2POW16_INV_2PI));
-    const float s = ieee::fsqrt(ieee::fmul(-2.0f, ieee::logf_(u)));
-    float       sv, cv;
-    ieee::sincosf_(a, &sv, &cv);
-    r[0] = __float2half_rn(ieee::fmul(sv, s));
-    r[1] = __float2half_rn(ieee::fmul(cv, s));
 }
 
 // rocrand_normal.h:196-220 roc_d_erfinv (host branch).
@@ -220,31 +358,29 @@ struct FnHalf // uniform_distribution<half> (uniform.hpp:105-117)
     }
 };
 
-struct FnNormalF // normal_distribution<float, uint, 4> (normal.hpp:49-69)
+// normal_distribution<float, uint, 4> (normal.hpp:49-69) and log_normal_distribution<float,
+// uint, 4> (log_normal.hpp:51-71)
+template<bool kLog>
+struct FnBoxMullerF
 {
     using T                      = float;
     static constexpr unsigned iw = 2, ow = 2;
+    static constexpr bool     kPair = true;
     float                     mean, stddev;
+    RB_HD static constexpr bool exponential() { return kLog; }
+    RB_HD nm::F2 uniforms(const uint32_t* a, const uint32_t* b) const { return uniform_pair(a[0], b[0]); }
+    RB_HD nm::F2 angles(const uint32_t* a, const uint32_t* b) const { return angle_pair(a[1], b[1]); }
+    RB_HD void   pair(const uint32_t* in0, const uint32_t* in1, T* out0, T* out1) const
+    {
+        normal_pair(*this, in0, in1, out0, out1);
+    }
     RB_HD void operator()(const uint32_t* in, T* out) const
     {
-        const float2 v = box_muller_f32(in[0], in[1]);
-        out[0]         = ieee::fadd(mean, ieee::fmul(v.x, stddev));
-        out[1]         = ieee::fadd(mean, ieee::fmul(v.y, stddev));
+        normal_unit(*this, in, out);
     }
 };
-
-struct FnLogNormalF // log_normal_distribution<float, uint, 4> (log_normal.hpp:51-71)
-{
-    using T                      = float;
-    static constexpr unsigned iw = 2, ow = 2;
-    float                     mean, stddev;
-    RB_HD void operator()(const uint32_t* in, T* out) const
-    {
-        const float2 v = box_muller_f32(in[0], in[1]);
-        out[0]         = ieee::expf_(ieee::fadd(mean, ieee::fmul(v.x, stddev)));
-        out[1]         = ieee::expf_(ieee::fadd(mean, ieee::fmul(v.y, stddev)));
-    }
-};
+using FnNormalF    = FnBoxMullerF<false>;
+using FnLogNormalF = FnBoxMullerF<true>;
 
 struct FnNormalD // normal_distribution<double, uint, 4> (normal.hpp:90-111)
 {
@@ -272,33 +408,35 @@ struct FnLogNormalD // log_normal_distribution<double, uint, 4> (log_normal.hpp:
     }
 };
 
-struct FnNormalH // normal_distribution<half, uint, 4> (normal.hpp:113-136), float branch
+// normal_distribution<half, uint, 4> (normal.hpp:113-136) and log_normal_distribution<half,
+// uint, 4> (log_normal.hpp:115-139), float branch
+template<bool kLog>
+struct FnBoxMullerH
 {
     using T                      = __half;
     static constexpr unsigned iw = 1, ow = 2;
+    static constexpr bool     kPair = true;
     float                     mean, stddev; // the half parameters widened to float
+    RB_HD static constexpr bool exponential() { return kLog; }
+    RB_HD nm::F2 uniforms(const uint32_t* a, const uint32_t* b) const
+    {
+        return uniform_pair_f16(a[0] & 0xffffu, b[0] & 0xffffu);
+    }
+    RB_HD nm::F2 angles(const uint32_t* a, const uint32_t* b) const
+    {
+        return angle_pair_f16(a[0] >> 16, b[0] >> 16);
+    }
+    RB_HD void pair(const uint32_t* in0, const uint32_t* in1, T* out0, T* out1) const
+    {
+        normal_pair(*this, in0, in1, out0, out1);
+    }
     RB_HD void operator()(const uint32_t* in, T* out) const
     {
-        __half r[2];
-        box_muller_f16(in[0], r);
-        out[0] = __float2half_rn(ieee::fadd(mean, ieee::fmul(stddev, __half2float(r[0]))));
-        out[1] = __float2half_rn(ieee::fadd(mean, ieee::fmul(stddev, __half2float(r[1]))));
+        normal_unit(*this, in, out);
     }
 };
-
-struct FnLogNormalH // log_normal_distribution<half, uint, 4> (log_normal.hpp:115-139)
-{
-    using T                      = __half;
-    static constexpr unsigned iw = 1, ow = 2;
-    float                     mean, stddev;
-    RB_HD void operator()(const uint32_t* in, T* out) const
-    {
-        __half r[2];
-        box_muller_f16(in[0], r);
-        out[0] = __float2half_rn(ieee::expf_(ieee::fadd(mean, ieee::fmul(stddev, __half2float(r[0])))));
-        out[1] = __float2half_rn(ieee::expf_(ieee::fadd(mean, ieee::fmul(stddev, __half2float(r[1])))));
-    }
-};
+using FnNormalH    = FnBoxMullerH<false>;
+using FnLogNormalH = FnBoxMullerH<true>;
 
 // poisson_distribution<ALIAS> (poisson.hpp:49-76).  The table is staged in shared memory
 // by the kernel; prob/alias then point there.
@@ -391,15 +529,25 @@ struct Fn64NormalF // box_muller(unsigned long long): x = low word, y = high wor
 {
     using T                      = float;
     static constexpr unsigned iw = 1, ow = 2;
+    static constexpr bool     kPair = true;
     float                     mean, stddev;
     bool                      log_normal;
+    RB_HD bool   exponential() const { return log_normal; }
+    RB_HD nm::F2 uniforms(const unsigned long long* a, const unsigned long long* b) const
+    {
+        return uniform_pair(static_cast<uint32_t>(a[0]), static_cast<uint32_t>(b[0]));
+    }
+    RB_HD nm::F2 angles(const unsigned long long* a, const unsigned long long* b) const
+    {
+        return angle_pair(static_cast<uint32_t>(a[0] >> 32), static_cast<uint32_t>(b[0] >> 32));
+    }
+    RB_HD void pair(const unsigned long long* in0, const unsigned long long* in1, T* out0, T* out1) const
+    {
+        normal_pair(*this, in0, in1, out0, out1);
+    }
     RB_HD void operator()(const unsigned long long* in, T* out) const
     {
-        const float2 v = box_muller_f32(static_cast<uint32_t>(in[0]), static_cast<uint32_t>(in[0] >> 32));
-        const float  a = ieee::fadd(mean, ieee::fmul(v.x, stddev));
-        const float  b = ieee::fadd(mean, ieee::fmul(v.y, stddev));
-        out[0]         = log_normal ? ieee::expf_(a) : a;
-        out[1]         = log_normal ? ieee::expf_(b) : b;
+        normal_unit(*this, in, out);
     }
 };
 
@@ -424,20 +572,26 @@ struct Fn64NormalH // normal_distribution_half2(ull): (ushort)v and (ushort)(v >
 {
     using T                      = __half;
     static constexpr unsigned iw = 1, ow = 2;
+    static constexpr bool     kPair = true;
     float                     mean, stddev;
     bool                      log_normal;
+    RB_HD bool   exponential() const { return log_normal; }
+    RB_HD nm::F2 uniforms(const unsigned long long* a, const unsigned long long* b) const
+    {
+        return uniform_pair_f16(static_cast<uint32_t>(a[0]) & 0xffffu, static_cast<uint32_t>(b[0]) & 0xffffu);
+    }
+    RB_HD nm::F2 angles(const unsigned long long* a, const unsigned long long* b) const
+    {
+        return angle_pair_f16(static_cast<uint32_t>(a[0] >> 32) & 0xffffu,
+                              static_cast<uint32_t>(b[0] >> 32) & 0xffffu);
+    }
+    RB_HD void pair(const unsigned long long* in0, const unsigned long long* in1, T* out0, T* out1) const
+    {
+        normal_pair(*this, in0, in1, out0, out1);
+    }
     RB_HD void operator()(const unsigned long long* in, T* out) const
     {
-        __half         r[2];
-        const uint32_t v = (static_cast<uint32_t>(in[0]) & 0xffffu)
-                           | (static_cast<uint32_t>(in[0] >> 32) << 16);
-        box_muller_f16(v, r);
-#pragma unroll
-        for(int k = 0; k < 2; k++)
-        {
-            const float z = ieee::fadd(mean, ieee::fmul(stddev, __half2float(r[k])));
-            out[k]        = __float2half_rn(log_normal ? ieee::expf_(z) : z);
-        }
+        normal_unit(*this, in, out);
     }
 };
 
@@ -527,11 +681,17 @@ struct FnMrgRemap // uint/uchar/ushort/half/Poisson: remap to [0, 2^32) then the
 {
     using T                      = typename Inner::T;
     static constexpr unsigned iw = 1, ow = Inner::ow;
+    static constexpr bool     kPair = has_pair<Inner>::value;
     Inner                     inner;
     RB_HD void operator()(const uint32_t* in, T* out) const
     {
         const uint32_t v = mrg_to_u32<N>(in[0]);
         inner(&v, out);
+    }
+    RB_HD void pair(const uint32_t* in0, const uint32_t* in1, T* out0, T* out1) const
+    {
+        const uint32_t v[2] = {mrg_to_u32<N>(in0[0]), mrg_to_u32<N>(in1[0])};
+        apply_pair(inner, v, v + 1, out0, out1);
     }
 };
 
@@ -562,19 +722,25 @@ struct FnMrgNormalF // mrg_box_muller (rocrand_normal.h:138-152)
 {
     using T                      = float;
     static constexpr unsigned iw = 2, ow = 2;
+    static constexpr bool     kPair = true;
     float                     mean, stddev;
     bool                      log_normal;
+    RB_HD bool   exponential() const { return log_normal; }
+    RB_HD nm::F2 uniforms(const uint32_t* a, const uint32_t* b) const
+    {
+        return nm::pack(mrg_to_f32<N>(a[0]), mrg_to_f32<N>(b[0]));
+    }
+    RB_HD nm::F2 angles(const uint32_t* a, const uint32_t* b) const
+    {
+        return nm::mul(nm::pack(mrg_to_f32<N>(a[1]), mrg_to_f32<N>(b[1])), nm::rep(6.2831855f));
+    }
+    RB_HD void pair(const uint32_t* in0, const uint32_t* in1, T* out0, T* out1) const
+    {
+        normal_pair(*this, in0, in1, out0, out1);
+    }
     RB_HD void operator()(const uint32_t* in, T* out) const
     {
-        const float u = mrg_to_f32<N>(in[0]);
-        const float v = ieee::fmul(mrg_to_f32<N>(in[1]), 6.2831855f);
-        const float s = ieee::fsqrt(ieee::fmul(-2.0f, ieee::logf_(u)));
-        float       sv, cv;
-        ieee::sincosf_(v, &sv, &cv);
-        const float a = ieee::fadd(mean, ieee::fmul(ieee::fmul(sv, s), stddev));
-        const float b = ieee::fadd(mean, ieee::fmul(ieee::fmul(cv, s), stddev));
-        out[0]        = log_normal ? ieee::expf_(a) : a;
-        out[1]        = log_normal ? ieee::expf_(b) : b;
+        normal_unit(*this, in, out);
     }
 };
 
@@ -611,19 +777,10 @@ struct FnMrgPoissonHuge
     }
 };
 
-// Transforms long enough (Box-Muller: a logarithm, a square root and a sine/cosine per
-// pair) that a thread gains from running two units side by side: MTGP32's fill takes two
-// units per step of its main loop for these.
+// Transforms that a thread runs several units of side by side: the packed fp32 / half pairs,
+// and the fp64 Box-Muller (a logarithm, a square root and a sine / cosine per unit).
 template<class F>
-struct long_transform : std::false_type
-{
-};
-template<>
-struct long_transform<FnNormalF> : std::true_type
-{
-};
-template<>
-struct long_transform<FnLogNormalF> : std::true_type
+struct long_transform : has_pair<F>
 {
 };
 template<>

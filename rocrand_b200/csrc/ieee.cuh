@@ -47,21 +47,11 @@ RB_HD double ull2d(unsigned long long v) { RB_PICK(__ull2double_rn(v), static_ca
 RB_HD uint32_t d2u_rz(double v) { RB_PICK(__double2uint_rz(v), static_cast<uint32_t>(v)); }
 RB_HD float d2f(double v) { RB_PICK(__double2float_rn(v), static_cast<float>(v)); }
 
-// The transcendental functions of the fp32 transforms: the device's own library functions
-// on the device (within an ulp or two of the host's), the C library's on the host (the
-// functions the reference's host generators call, so the host path is bit-exact).
-RB_HD float logf_(float x) { RB_PICK(logf(x), std::log(x)); }
+// The exponential of the log-normal transforms: the device's own library function on the
+// device (within an ulp or two of the host's), the C library's on the host (the function the
+// reference's host generators call, so the host path is bit-exact).
 RB_HD float expf_(float x) { RB_PICK(expf(x), std::exp(x)); }
 RB_HD double exp_(double x) { RB_PICK(exp(x), std::exp(x)); }
-RB_HD void sincosf_(float x, float* s, float* c)
-{
-#if defined(__CUDA_ARCH__)
-    sincosf(x, s, c);
-#else
-    *s = std::sin(x);
-    *c = std::cos(x);
-#endif
-}
 
 } // namespace ieee
 } // namespace rb200

@@ -446,10 +446,8 @@ constexpr bool kMtStaged = std::is_same<F, FnNormalD>::value || std::is_same<F, 
                            || std::is_same<F, FnNormalH>::value || std::is_same<F, FnLogNormalH>::value;
 
 // Units a lane transforms side by side in a staged round inside the call: four fp64
-// Box-Muller chains, three fp32 / half ones.
-template<class F>
-constexpr unsigned kMtUnitsPerStep
-    = (std::is_same<F, FnNormalD>::value || std::is_same<F, FnLogNormalD>::value) ? 4u : 3u;
+// Box-Muller chains, two packed pairs of fp32 or half ones.
+constexpr unsigned kMtUnitsPerStep = 4;
 
 // Shared memory of one block of mt_fill: the distribution's table, or the staged state.
 template<class F>
@@ -511,16 +509,13 @@ __device__ __forceinline__ void round_edge(const U& u, const MtArgs& a, long lon
         ...);
 }
 
-// One input unit of a staged round: tempered slots G*iw .. G*iw+iw-1 through F.
+// Inputs of one unit of a staged round: tempered slots G*iw .. G*iw+iw-1.
 template<class F>
-__device__ __forceinline__ void staged_unit(const F& f, const uint32_t* s, unsigned G,
-                                            typename F::T (&out)[F::ow])
+__device__ __forceinline__ void staged_inputs(const uint32_t* s, unsigned G, uint32_t (&in)[F::iw])
 {
-    uint32_t in[F::iw];
 #pragma unroll
     for(unsigned i = 0; i < F::iw; i++)
         in[i] = mt_temper(s[(G * F::iw + i) * kMtBlock]);
-    f(in, out);
 }
 
 // A round whose slots were staged in shared memory (slot j of this thread at s[j * 64]):
@@ -541,15 +536,19 @@ __device__ __forceinline__ void mt_round_staged(const F& f, const uint32_t* s, c
     const long long    q0   = base + tid;
     if(base >= 0 && static_cast<unsigned long long>(base) + a.full <= a.total)
     {
-        constexpr unsigned U = kMtUnitsPerStep<F>;
+        constexpr unsigned U = kMtUnitsPerStep;
         unsigned           G = 0;
 #pragma unroll 1
         for(; G + U <= per; G += U)
         {
-            T o[U][ow];
+            uint32_t in[U][F::iw];
+            T        o[U][ow];
 #pragma unroll
             for(unsigned u = 0; u < U; u++)
-                staged_unit(f, s, G + u, o[u]);
+                staged_inputs<F>(s, G + u, in[u]);
+#pragma unroll
+            for(unsigned u = 0; u < U; u += 2)
+                apply_pair(f, in[u], in[u + 1], o[u], o[u + 1]);
 #pragma unroll
             for(unsigned u = 0; u < U; u++)
                 store_vec(a.vec + static_cast<unsigned long long>(q0 + (G + u) * kMtThreads) * VB, o[u]);
@@ -557,8 +556,10 @@ __device__ __forceinline__ void mt_round_staged(const F& f, const uint32_t* s, c
 #pragma unroll 1
         for(; G < per; G++)
         {
-            T o0[ow];
-            staged_unit(f, s, G, o0);
+            uint32_t in[F::iw];
+            T        o0[ow];
+            staged_inputs<F>(s, G, in);
+            f(in, o0);
             store_vec(a.vec + static_cast<unsigned long long>(q0 + G * kMtThreads) * VB, o0);
         }
         return;
@@ -569,8 +570,10 @@ __device__ __forceinline__ void mt_round_staged(const F& f, const uint32_t* s, c
         const long long q = q0 + static_cast<long long>(G) * kMtThreads;
         if(q < 0 || static_cast<unsigned long long>(q) >= a.total)
             continue;
-        T out[ow];
-        staged_unit(f, s, G, out);
+        uint32_t in[F::iw];
+        T        out[ow];
+        staged_inputs<F>(s, G, in);
+        f(in, out);
         if(static_cast<unsigned long long>(q) < a.vec_n)
         {
             store_vec(a.vec + static_cast<unsigned long long>(q) * VB, out);

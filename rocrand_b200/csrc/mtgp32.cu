@@ -56,8 +56,8 @@ struct MtgpArgs
     uint32_t           head, tail;
 };
 
-// Units a thread transforms side by side in the main loop: four fp64 Box-Muller chains,
-// two fp32 ones.
+// Units a thread transforms side by side in the main loop: four fp64 Box-Muller chains, one
+// packed pair of fp32 or half ones.
 template<class F>
 constexpr unsigned kMtgpUnits
     = (std::is_same<F, FnNormalD>::value || std::is_same<F, FnLogNormalD>::value) ? 4u : 2u;
@@ -131,8 +131,8 @@ __global__ void __launch_bounds__(kMtgpBlock, 4) mtgp_fill(MtgpArgs a, F fw)
                     in[u][i] = step();
             T o[U][ow];
 #pragma unroll
-            for(unsigned u = 0; u < U; u++)
-                f(in[u], o[u]);
+            for(unsigned u = 0; u < U; u += 2)
+                apply_pair(f, in[u], in[u + 1], o[u], o[u + 1]);
 #pragma unroll
             for(unsigned u = 0; u < U; u++)
                 store_small(a.vec + (index + u * str) * VB, o[u]);

@@ -195,8 +195,27 @@ __global__ void __launch_bounds__(kBlock) stateful_fill(FillArgs a, F f)
     uint32_t           in[F::iw];
     T                  out[F::ow];
     unsigned long long j = t;
-    // unrolled so that the state words rotate back into place (no register moves per step)
+    if constexpr(has_pair<F>::value)
+    {
+        // two vectors' units side by side
 #pragma unroll(E::kUnroll)
+        for(; j + kE < a.vec_n; j += 2 * kE)
+        {
+            uint32_t in1[F::iw];
+            T        out1[F::ow];
+#pragma unroll
+            for(unsigned i = 0; i < F::iw; i++)
+                in[i] = eng.next();
+#pragma unroll
+            for(unsigned i = 0; i < F::iw; i++)
+                in1[i] = eng.next();
+            g.pair(in, in1, out, out1);
+            store_small(a.vec + j * VB, out);
+            store_small(a.vec + (j + kE) * VB, out1);
+        }
+    }
+    // unrolled so that the state words rotate back into place (no register moves per step)
+#pragma unroll(has_pair<F>::value ? 1 : E::kUnroll)
     for(; j < a.vec_n; j += kE)
     {
 #pragma unroll

@@ -264,6 +264,24 @@ __device__ __forceinline__ void store_vec(unsigned char* p, const T (&v)[N])
     }
 }
 
+// The units of one block of words, two at a time where there are two.
+template<class W, int D, class F>
+__device__ __forceinline__ void tf_units(const F& f, const TfBlock<W, D>& b,
+                                         typename F::T (&out)[D / F::iw * F::ow])
+{
+    constexpr unsigned opt = D / F::iw;
+    if constexpr(opt == 1)
+    {
+        f(b.w, out);
+    }
+    else
+    {
+#pragma unroll
+        for(unsigned s = 0; s < opt; s += 2)
+            apply_pair(f, b.w + s * F::iw, b.w + (s + 1) * F::iw, out + s * F::ow, out + (s + 1) * F::ow);
+    }
+}
+
 template<class W, int D, class F, bool kAligned>
 __global__ void __launch_bounds__(kBlock) threefry_fill(TfCall<W, D> a, F f)
 {
@@ -275,7 +293,22 @@ __global__ void __launch_bounds__(kBlock) threefry_fill(TfCall<W, D> a, F f)
     const unsigned long long tid    = static_cast<unsigned long long>(blockIdx.x) * kBlock + threadIdx.x;
     const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * kBlock;
 
-    for(unsigned long long j = tid; j < a.vec_n; j += stride)
+    unsigned long long j = tid;
+    if constexpr(kAligned && opt == 1 && has_pair<F>::value)
+    {
+        // one unit per vector (2x32): the units of two vectors side by side
+        for(; j + stride < a.vec_n; j += 2 * stride)
+        {
+            const unsigned long long q  = (a.s0 + a.adj) / D + j;
+            const TfBlock<W, D>      b0 = threefry_block(tf_add(a.c0, q), a.keys);
+            const TfBlock<W, D>      b1 = threefry_block(tf_add(a.c0, q + stride), a.keys);
+            typename F::T            out0[F::ow], out1[F::ow];
+            g.pair(b0.w, b1.w, out0, out1);
+            store_vec(a.vec + j * VB, out0);
+            store_vec(a.vec + (j + stride) * VB, out1);
+        }
+    }
+    for(; j < a.vec_n; j += stride)
     {
         TfBlock<W, D> b;
         if(kAligned)
@@ -292,9 +325,7 @@ __global__ void __launch_bounds__(kBlock) threefry_fill(TfCall<W, D> a, F f)
                 b = tf_interleave(b, threefry_block(tf_add(c, 1), a.keys), s);
         }
         typename F::T out[opt * F::ow];
-#pragma unroll
-        for(unsigned s = 0; s < opt; s++)
-            g(b.w + s * F::iw, out + s * F::ow);
+        tf_units(g, b, out);
         store_vec(a.vec + j * VB, out);
     }
 
