@@ -225,6 +225,16 @@ RB_HD void apply_pair(const F& f, const W* in0, const W* in1, typename F::T* out
     }
 }
 
+// mean + stddev v: one rounding on the device, the reference's two on the host.
+RB_HD double scaled_f64(double v, double stddev, double mean)
+{
+#if defined(__CUDA_ARCH__)
+    return __fma_rn(v, stddev, mean);
+#else
+    return mean + v * stddev;
+#endif
+}
+
 // rocrand_normal.h:68-89 (host branch: sin/cos of w * pi rounded in double).
 RB_HD double2 box_muller_f64(uint32_t x, uint32_t y, uint32_t z, uint32_t w)
 {
@@ -232,7 +242,7 @@ RB_HD double2 box_muller_f64(uint32_t x, uint32_t y, uint32_t z, uint32_t w)
     const double   u  = ieee::dfma(ieee::ull2d(v1), RB_2POW53_INV_DOUBLE, RB_2POW53_INV_DOUBLE);
     const uint64_t v2 = (uint64_t)z ^ ((uint64_t)w << 21);
     const double   ww = ieee::dfma(ieee::ull2d(v2), RB_2POW53_INV_DOUBLE * 2.0, RB_2POW53_INV_DOUBLE * 2.0);
-    const double   s  = ieee::dsqrt(ieee::dmul(-2.0, pm::log(u)));
+    const double   s  = pm::sqrt_inner(ieee::dmul(-2.0, pm::log_uniform(u)));
     const double   a  = ieee::dmul(ww, RB_PI_DOUBLE);
     double         sv, cv;
     pm::sincos(a, sv, cv);
@@ -390,8 +400,8 @@ struct FnNormalD // normal_distribution<double, uint, 4> (normal.hpp:90-111)
     RB_HD void operator()(const uint32_t* in, T* out) const
     {
         const double2 v = box_muller_f64(in[0], in[1], in[2], in[3]);
-        out[0]          = ieee::dadd(mean, ieee::dmul(v.x, stddev));
-        out[1]          = ieee::dadd(mean, ieee::dmul(v.y, stddev));
+        out[0]          = scaled_f64(v.x, stddev, mean);
+        out[1]          = scaled_f64(v.y, stddev, mean);
     }
 };
 
@@ -403,8 +413,8 @@ struct FnLogNormalD // log_normal_distribution<double, uint, 4> (log_normal.hpp:
     RB_HD void operator()(const uint32_t* in, T* out) const
     {
         const double2 v = box_muller_f64(in[0], in[1], in[2], in[3]);
-        out[0]          = ieee::exp_(ieee::dadd(mean, ieee::dmul(v.x, stddev)));
-        out[1]          = ieee::exp_(ieee::dadd(mean, ieee::dmul(v.y, stddev)));
+        out[0]          = ieee::exp_(scaled_f64(v.x, stddev, mean));
+        out[1]          = ieee::exp_(scaled_f64(v.y, stddev, mean));
     }
 };
 
@@ -561,8 +571,8 @@ struct Fn64NormalD // box_muller_double(ulonglong2)
     {
         const double2 v = box_muller_f64(static_cast<uint32_t>(in[0]), static_cast<uint32_t>(in[0] >> 32),
                                          static_cast<uint32_t>(in[1]), static_cast<uint32_t>(in[1] >> 32));
-        const double  a = ieee::dadd(mean, ieee::dmul(v.x, stddev));
-        const double  b = ieee::dadd(mean, ieee::dmul(v.y, stddev));
+        const double  a = scaled_f64(v.x, stddev, mean);
+        const double  b = scaled_f64(v.y, stddev, mean);
         out[0]          = log_normal ? ieee::exp_(a) : a;
         out[1]          = log_normal ? ieee::exp_(b) : b;
     }
@@ -755,11 +765,11 @@ struct FnMrgNormalD // mrg_box_muller_double (rocrand_normal.h:154-172): float u
     {
         const double u = (double)mrg_to_f32<N>(in[0]);
         const double v = (double)mrg_to_f32<N>(in[1]) * 2.0;
-        const double s = ieee::dsqrt(ieee::dmul(-2.0, pm::log(u)));
+        const double s = pm::sqrt_inner(ieee::dmul(-2.0, pm::log_uniform(u)));
         double       sv, cv;
         pm::sincos(ieee::dmul(v, RB_PI_DOUBLE), sv, cv);
-        const double a = ieee::dadd(mean, ieee::dmul(ieee::dmul(sv, s), stddev));
-        const double b = ieee::dadd(mean, ieee::dmul(ieee::dmul(cv, s), stddev));
+        const double a = scaled_f64(ieee::dmul(sv, s), stddev, mean);
+        const double b = scaled_f64(ieee::dmul(cv, s), stddev, mean);
         out[0]         = log_normal ? ieee::exp_(a) : a;
         out[1]         = log_normal ? ieee::exp_(b) : b;
     }

@@ -12,11 +12,21 @@
 //    r = z invc - 1 is exact in one fma (|r| < 2^-8; the subinterval around 1 has c = 1);
 //    log x = (k ln2_hi + log c_hi) + r - r^2/2 + r^3 P(r) + small terms, the first sums
 //    compensated and one final rounding;
-//  * sin/cos x (0 <= x <~ 8): x = k pi/2 + r (pi/2 in three parts), |r| = j/64 + b,
-//    sin/cos(j/64) from a double-double table, sin b and cos b - 1 by short series.
+//  * sin/cos x (0 <= x <= 2 pi): x = m C + b with C = 2 pi / 464 as a double, m the nearest;
+//    b is exact in one fma (x and m C are multiples of 2^-60 where m > 0, and |b| < 2^-7), so
+//    neither the reduction nor b needs a second word; sin/cos(m C) from a double-double table
+//    over the whole circle (15 KB, so no quadrant to select either); sin b and cos b - 1 by
+//    short series.
 // Both are IEEE operations only (add, mul, fma, sqrt-free), so host and device builds of
 // this header give identical results; the tables are computed in binary128 at build time
 // (rocrand_b200/data/make_precise_tables.c).
+// Issue bounds the transforms (an fp64 instruction takes two to three cycles of its scheduler:
+// 2.07 with constant operands, 3.03 with three registers, every other about one): a Philox
+// Box-Muller pair took 269 instructions, 108 of them fp64, with a two-step reduction (k pi/2 in
+// three parts, then j/64), the special cases of log in line and sqrt.rn; now 184 and 76.  Normal
+// fp64, 2^25 values a call on one B200, before -> now: Philox 191 -> 141 us, XORWOW 196 -> 139,
+// LFSR113 223 -> 161, MRG32k3a 234 -> 176, MT19937 263 -> 191, MTGP32 274 -> 232, ThreeFry4x64
+// 249 -> 206.  Misses of correct rounding in 3 10^6: sine 32 -> 27, cosine 23 -> 23, log 0.
 #pragma once
 
 #include "precise_tables.inc"
@@ -36,40 +46,27 @@ namespace rb200
 namespace pm
 {
 
+// rows of four doubles: (invc, head, tail, 0) and (sin hi, sin lo, cos hi, cos lo)
 #if defined(__CUDACC__)
-static __device__ const double kLogTabDev[RB_LOG_ROWS * 3] = RB_LOG_INIT;
-static __device__ const double kScTabDev[RB_SC_TABLE_ROWS * 4]    = RB_SC_TABLE_INIT;
-#endif
-static const double kLogTabHost[RB_LOG_ROWS * 3] = RB_LOG_INIT;
-static const double kScTabHost[RB_SC_TABLE_ROWS * 4]    = RB_SC_TABLE_INIT;
-
-RB_PM_HD const double* log_table()
+struct __align__(16) Row
 {
-#if defined(__CUDA_ARCH__)
-    return kLogTabDev;
-#else
-    return kLogTabHost;
+    double v0, v1, v2, v3;
+};
+static __device__ const Row kLogTabDev[RB_LOG_ROWS]     = RB_LOG_INIT;
+static __device__ const Row kScTabDev[RB_SC_TABLE_ROWS] = RB_SC_TABLE_INIT;
 #endif
-}
+static const double kLogTabHost[RB_LOG_ROWS][4]     = RB_LOG_INIT;
+static const double kScTabHost[RB_SC_TABLE_ROWS][4] = RB_SC_TABLE_INIT;
 
-RB_PM_HD const double* sc_table()
-{
+// Row i of a table, read as 16-byte halves through the non-coherent cache on the device.
 #if defined(__CUDA_ARCH__)
-    return kScTabDev;
+#define RB_PM_ROW(name, i, r)                                                        \
+    const double2 r##_a = __ldg(reinterpret_cast<const double2*>(name##Dev + (i)));  \
+    const double2 r##_b = __ldg(reinterpret_cast<const double2*>(name##Dev + (i)) + 1); \
+    const double  r[4]  = {r##_a.x, r##_a.y, r##_b.x, r##_b.y}
 #else
-    return kScTabHost;
+#define RB_PM_ROW(name, i, r) const double* const r = name##Host[i]
 #endif
-}
-
-// read-only table entry (through the non-coherent cache on the device)
-RB_PM_HD double tab(const double* p)
-{
-#if defined(__CUDA_ARCH__)
-    return __ldg(p);
-#else
-    return *p;
-#endif
-}
 
 RB_PM_HD double fma_(double a, double b, double c)
 {
@@ -109,27 +106,20 @@ RB_PM_HD void fast_two_sum(double a, double b, double& s, double& e)
     e = b - (s - a);
 }
 
-// Natural logarithm, near-correctly rounded.
-RB_PM_HD double log(double x)
+// Natural logarithm of a positive normal x, given by its bits, less `down` times ln 2.  (Any
+// bits give a table row in range: log() selects its special cases afterwards.)
+RB_PM_HD double log_core(uint64_t ix, int down)
 {
-    // The main path runs for every input (the special cases are selected at the end, so
-    // that independent calls can interleave): zero, negative, NaN and infinity still give
-    // a table row in range there.
-    const double x0  = x;
-    const bool   sub = x < 0x1p-1022; // subnormal (or zero / negative: replaced below)
-    x                = sub ? x * 0x1p54 : x;
-    const uint64_t ix  = bits_of(x);
     const uint64_t tmp = ix - RB_LOG_OFF;
     const unsigned i   = static_cast<unsigned>(tmp >> 44) & 255u;
-    const int      k   = static_cast<int>(static_cast<int64_t>(tmp) >> 52) - (sub ? 54 : 0);
+    const int      k   = static_cast<int>(static_cast<int64_t>(tmp) >> 52) - down;
     const double   z   = from_bits(ix - (tmp & 0xfff0000000000000ull)); // x / 2^k in [OFF, 2 OFF)
-    const double*  row = log_table() + 3 * i;
-    const double   invc = tab(row), lch = tab(row + 1), lcl = tab(row + 2);
-    const double   kd   = static_cast<double>(k);
-    const double   r    = fma_(z, invc, -1.0);       // exact: |r| < 2^-8, invc has <= 9 bits
-    const double   t1   = fma_(kd, RB_LN2_HI, lch);  // exact: both multiples of 2^-42, |t1| < 2^10
-    double         s1, e1, s2, e2;
-    two_sum(t1, r, s1, e1);
+    RB_PM_ROW(kLogTab, i, row);
+    const double kd = static_cast<double>(k);
+    const double r  = fma_(z, row[0], -1.0);          // exact: |r| < 2^-8, invc has <= 9 bits
+    const double t1 = fma_(kd, RB_LN2_HI, row[1]);    // exact: both multiples of 2^-42, |t1| < 2^10
+    double       s1, e1, s2, e2;
+    fast_two_sum(t1, r, s1, e1); // |t1| >= |r| or t1 = 0 (checked over the rows at build time)
     // -r^2 / 2 = q + ql exactly
     const double r2 = r * r;
     const double q  = -0.5 * r2;
@@ -145,68 +135,86 @@ RB_PM_HD double log(double x)
     p        = fma_(p, r, -1.0 / 4.0);
     p        = fma_(p, r, 1.0 / 3.0);
     const double tail = p * (r2 * r);
-    const double low  = ((e1 + e2) + (ql + lcl)) + fma_(kd, RB_LN2_LO, tail);
-    const double y    = s2 + low;
-    return x0 > 0.0 ? (x0 == INFINITY ? x0 : y) : (x0 == 0.0 ? -INFINITY : NAN);
+    const double low  = ((e1 + e2) + (ql + row[2])) + fma_(kd, RB_LN2_LO, tail);
+    return s2 + low;
 }
 
-// sin and cos of x for 0 <= x < 8 (the Box-Muller angles 0 .. 2 pi), near-correctly rounded.
+// Natural logarithm, near-correctly rounded.
+RB_PM_HD double log(double x)
+{
+    const bool   sub = x < 0x1p-1022; // subnormal (or zero / negative: replaced below)
+    const double y   = log_core(bits_of(sub ? x * 0x1p54 : x), sub ? 54 : 0);
+    return x > 0.0 ? (x == INFINITY ? x : y) : (x == 0.0 ? -INFINITY : NAN);
+}
+
+// The same for a uniform, 2^-1022 <= x <= 1: no special case.
+RB_PM_HD double log_uniform(double x)
+{
+    return log_core(bits_of(x), 0);
+}
+
+// sin and cos of x for 0 <= x <= 2 pi (the Box-Muller angles; 2 pi as a double), near-correctly
+// rounded.
 RB_PM_HD void sincos(double x, double& s_out, double& c_out)
 {
-    const double kd = rint(x * RB_2_OVER_PI);
-    const int    k  = static_cast<int>(kd);
-    // r = x - k pi/2 as rh + rl (k pi/2 in three parts; the first two products are exact)
-    const double t  = fma_(-kd, RB_PIO2_1, x);
-    const double p2 = kd * RB_PIO2_2;
-    double       rh, rl;
-    two_sum(t, -p2, rh, rl);
-    rl = fma_(-kd, RB_PIO2_3, rl);
-    {
-        const double h = rh + rl;
-        rl             = rl - (h - rh);
-        rh             = h;
-    }
-    const bool neg = rh < 0.0;
-    rh             = neg ? -rh : rh;
-    rl             = neg ? -rl : rl;
-    const int     j   = static_cast<int>(rint(rh * 64.0));
-    const double* row = sc_table() + 4 * j;
-    const double  sh = tab(row), sl = tab(row + 1), ch = tab(row + 2), cl = tab(row + 3);
-    const double  bh = rh - static_cast<double>(j) * (1.0 / 64.0); // exact
-    const double  bl = rl;
-    const double  b2 = bh * bh;
-    // sin b - bh = bl + bh^3 (-1/6 + b^2/120 - b^4/5040);  cos b - 1 = -b^2/2 + b^4 (1/24 -
-    // b^2/720); |b| <= 2^-7, the first terms left out (b^9/9!, b^8/8!) are below 2^-71
+    // m = x / C rounded, as the low bits of t = 1.5 2^52 + m and as a double
+    const double t  = fma_(x, RB_SC_INV_STEP, 0x1.8p52);
+    const double md = t - 0x1.8p52;
+    const int    m  = static_cast<int>(static_cast<uint32_t>(bits_of(t)));
+    RB_PM_ROW(kScTab, m, row);
+    const double sh = row[0], sl = row[1], ch = row[2], cl = row[3];
+    const double b  = fma_(md, -RB_SC_STEP, x); // exact, |b| < 2^-7
+    const double b2 = b * b;
+    // sin b - b = b^3 (-1/6 + b^2/120 - b^4/5040);  cos b - 1 = b^2 (-1/2 + b^2/24 - b^4/720);
+    // the first terms left out (b^9/9!, b^8/8!) are below 2^-73 of b and of 1
     double sp = -1.0 / 5040.0;
     sp        = fma_(sp, b2, 1.0 / 120.0);
     sp        = fma_(sp, b2, -1.0 / 6.0);
-    const double sinb_rest = fma_(sp * b2, bh, bl); // bl + bh^3 S(b^2)
+    const double sinb_rest = (sp * b2) * b;
     double       cp        = -1.0 / 720.0;
     cp                     = fma_(cp, b2, 1.0 / 24.0);
-    // cos b - 1 = -b^2/2 + b^4 C(b^2), with b^2 including the low part of b
-    const double bb  = fma_(2.0 * bh, bl, b2);
-    const double cm1 = fma_(cp * bb, bb, -0.5 * bb);
+    cp                     = fma_(cp, b2, -0.5);
+    const double cm1 = cp * b2;
     // sin(a + b) = sin a + (cos a * b + sin a * (cos b - 1) + cos a * (sin b - b))
-    const double psh = ch * bh;
-    const double psl = fma_(ch, bh, -psh);
+    const double psh = ch * b;
+    const double psl = fma_(ch, b, -psh);
     double       ssh, ssl;
-    fast_two_sum(sh, psh, ssh, ssl); // sin a >= sin(1/64) > |cos a * b| unless a = 0
-    const double s_low = ((ssl + psl) + sl) + fma_(cl, bh, fma_(sh, cm1, ch * sinb_rest));
-    const double sv    = ssh + s_low;
+    // |sin a| >= sin C > |cos a * b|, or sin a = 0: the rows at the multiples of pi, where it
+    // is below 2^-57, have it in their low word alone
+    fast_two_sum(sh, psh, ssh, ssl);
+    const double s_low = ((ssl + psl) + sl) + fma_(cl, b, fma_(sh, cm1, ch * sinb_rest));
+    s_out              = ssh + s_low;
     // cos(a + b) = cos a - (sin a * b) + cos a * (cos b - 1) - sin a * (sin b - b)
-    const double pch = sh * bh;
-    const double pcl = fma_(sh, bh, -pch);
+    const double pch = sh * b;
+    const double pcl = fma_(sh, b, -pch);
     double       csh, csl;
-    fast_two_sum(ch, -pch, csh, csl); // cos a >= 0.7 > |sin a * b|
-    const double c_low = ((csl - pcl) + cl) + fma_(-sl, bh, fma_(ch, cm1, -(sh * sinb_rest)));
-    const double cv    = csh + c_low;
-    const double s     = neg ? -sv : sv;
-    // quadrant k: (sin, cos) = (s, c), (c, -s), (-s, -c), (-c, s)
-    const bool   odd   = (k & 1) != 0;
-    const double so    = odd ? cv : s;
-    const double co    = odd ? s : cv;
-    s_out              = (k & 2) ? -so : so;
-    c_out              = ((k + 1) & 2) ? -co : co;
+    fast_two_sum(ch, -pch, csh, csl); // likewise
+    const double c_low = ((csl - pcl) + cl) + fma_(-sl, b, fma_(ch, cm1, -(sh * sinb_rest)));
+    c_out              = csh + c_low;
+}
+
+// Square root of t = 0 or 2^-200 <= t <= 2^200, correctly rounded but for near-halfway cases
+// within 2^-100 relative: the hardware's 20-bit reciprocal square root y, one third-order step
+// on t y and y / 2, and Markstein's residual correction.  (sqrt.rn's range check and its out of
+// line path are what this saves: the same number of fp64 operations.)
+RB_PM_HD double sqrt_inner(double t)
+{
+#if defined(__CUDA_ARCH__)
+    // t = 0 seeds with a tiny number instead, and t y = 0 then stays 0
+    const double seed = __hiloint2double(max(__double2hiint(t), 0x02000000), __double2loint(t));
+    double       y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(seed));
+    const double g  = t * y;
+    const double h  = 0.5 * y;
+    const double e  = fma_(-g, h, 0.5);
+    const double q  = e * fma_(1.5, e, 1.0);
+    const double g1 = fma_(g, q, g);
+    const double h1 = fma_(h, q, h);
+    const double r  = fma_(-g1, g1, t);
+    return fma_(r, h1, g1);
+#else
+    return std::sqrt(t);
+#endif
 }
 
 // Natural logarithm of a float, correctly rounded except in rare double-rounding cases.

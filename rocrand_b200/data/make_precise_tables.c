@@ -11,11 +11,14 @@
  *    one fma; the subinterval holding 1.0 takes c = 1.  -log(invc_i) is stored as a head
  *    rounded to a multiple of 2^-42 and a tail, so k ln2_hi + head is exact;
  *    ln 2 as a 42-bit head (exact times any exponent) and a tail;
- *  * sincos: for j = 0..51, sin(j/64) and cos(j/64) as (hi, lo) pairs;  pi/2 as three
- *    parts of 40, 40 and 53 bits, and 2/pi.
+ *  * sincos: for m = 0..464, sin(m C) and cos(m C), C = 2 pi / 464 as a double, as (hi, lo)
+ *    pairs; at the multiples of pi/2 the one that is only C's rounding error is all low word.
+ *    (464 C is within 5e-18 of 2 pi, which no power of two of divisions gives: the kernels
+ *    leave out that error's product with cos b - 1.)
  *
  * Usage: make_precise_tables <output.inc>
  */
+#include <math.h>
 #include <quadmath.h>
 #include <stdio.h>
 #include <string.h>
@@ -43,7 +46,7 @@ int main(int argc, char** argv)
         return 1;
     }
     fprintf(f, "/* generated by rocrand_b200/data/make_precise_tables.c */\n");
-    /* log table of the offset split: rows (invc, -log(invc) head, tail), i = 0..255 */
+    /* log table of the offset split: rows (invc, -log(invc) head, tail, 0), i = 0..255 */
     {
         const unsigned long long off = 0x3FE6A80000000000ull;
         fprintf(f, "#define RB_LOG_OFF 0x%016llxull\n#define RB_LOG_ROWS 256\n", off);
@@ -81,7 +84,14 @@ int main(int argc, char** argv)
             const __float128 l  = -logq((__float128)invc);
             const double     hi = (double)(rintq(ldexpq(l, 42)) / 0x1p42Q);
             const double     lo = (double)(l - (__float128)hi);
-            fprintf(f, "    %a, %a, %a, \\\n", invc, hi, lo);
+            /* the kernels' first sum takes |head| >= |r| (or a zero head) for granted; with
+               k ln 2 added it holds by far */
+            if(hi != 0.0 && (fabs(hi) < fabsq(rl) || fabs(hi) < fabsq(rh)))
+            {
+                fprintf(stderr, "log table row %u: |head| < |r|\n", i);
+                return 1;
+            }
+            fprintf(f, "    {%a, %a, %a, 0.0}, \\\n", invc, hi, lo);
         }
         fprintf(f, "}\n");
     }
@@ -140,23 +150,19 @@ int main(int argc, char** argv)
         const float  l2fl = (float)(ln2 - (__float128)l2fh);
         fprintf(f, "#define RB_LN2F_HI %af\n#define RB_LN2F_LO %af\n", l2fh, (double)l2fl);
     }
-    /* sincos table: rows (sin hi, sin lo, cos hi, cos lo) at j/64, j = 0..51 */
-    fprintf(f, "#define RB_SC_TABLE_ROWS 52\n#define RB_SC_TABLE_INIT { \\\n");
-    for(int j = 0; j <= 51; j++)
+    /* sincos table: rows (sin hi, sin lo, cos hi, cos lo) at m C, m = 0..464 */
+    const double step = (double)(2.0Q * M_PIq / 464.0Q);
+    fprintf(f, "#define RB_SC_STEP %a\n#define RB_SC_INV_STEP %a\n", step, (double)(1.0Q / (__float128)step));
+    fprintf(f, "#define RB_SC_TABLE_ROWS 465\n#define RB_SC_TABLE_INIT { \\\n");
+    for(int m = 0; m <= 464; m++)
     {
-        const __float128 a  = (__float128)j / 64.0Q;
+        const __float128 a  = (__float128)m * (__float128)step; /* exact: 53 + 9 bits */
         const __float128 s  = sinq(a), c = cosq(a);
-        const double     sh = (double)s, ch = (double)c;
-        fprintf(f, "    %a, %a, %a, %a, \\\n", sh, (double)(s - (__float128)sh), ch,
+        const double     sh = m % 232 == 0 ? 0.0 : (double)s, ch = m % 232 == 116 ? 0.0 : (double)c;
+        fprintf(f, "    {%a, %a, %a, %a}, \\\n", sh, (double)(s - (__float128)sh), ch,
                 (double)(c - (__float128)ch));
     }
     fprintf(f, "}\n");
-    const __float128 pio2 = acosq(0.0Q);
-    const double     p1   = round_bits(pio2, 40);
-    const double     p2   = round_bits(pio2 - (__float128)p1, 40);
-    const double     p3   = (double)(pio2 - (__float128)p1 - (__float128)p2);
-    fprintf(f, "#define RB_PIO2_1 %a\n#define RB_PIO2_2 %a\n#define RB_PIO2_3 %a\n", p1, p2, p3);
-    fprintf(f, "#define RB_2_OVER_PI %a\n", (double)(1.0Q / pio2));
     if(fclose(f) != 0)
     {
         perror(argv[1]);
