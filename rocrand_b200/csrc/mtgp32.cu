@@ -13,7 +13,7 @@
 //
 // B200 layout: the rings and offsets of the 512 generators live in HBM (2 MiB); each block
 // keeps its ring in shared memory for the whole call (one __syncthreads per step: a step's
-// reads stop 1 short of its first write, the next step reads what it wrote), its parameter
+// reads stop short of its first write, the next step reads what it wrote), its parameter
 // set in registers and shared memory.  The parameter sets are the published MTGP32 11213
 // dynamic-creator sets (rocrand_b200/data/mtgp32_params.bin, embedded by mtgp32_data.S).
 #include "common.hpp"
@@ -56,25 +56,44 @@ struct MtgpArgs
     uint32_t           head, tail;
 };
 
-// Units a thread transforms side by side in the main loop: four fp64 Box-Muller chains, one
-// packed pair of fp32 or half ones.
+// Units a thread takes in one iteration of the main loop: whole turns of four block steps, and
+// for the long transforms the units they run side by side (four fp64 Box-Muller chains, packed
+// pairs of fp32 or half ones).
 template<class F>
-constexpr unsigned kMtgpUnits
-    = (std::is_same<F, FnNormalD>::value || std::is_same<F, FnLogNormalD>::value) ? 4u : 2u;
+constexpr unsigned kMtgpUnits = F::iw == 1 ? 4u : F::iw == 2 ? 2u : 4u;
 
-// 4 blocks of 256 threads per SM (at most 64 registers): all 512 block generators resident
-// at once on 148 SMs.
+// Words after the ring that repeat its first ones: a step reads up to pos + 255 words ahead of
+// its offset, pos <= kMtgpReach, the last of the four offsets being 768.
+constexpr int kMtgpReach  = 95;
+constexpr int kMtgpMirror = 96;
+static_assert(kMtgpBlock + kMtgpReach <= kMtgpN, "a step reads no word that it writes");
+
+// The ring in shared memory starts at the call's offset, so that the four block steps of a turn
+// work at the constant offsets 0, 256, 512 and 768 and every address is the thread's base plus
+// an immediate.  Only step 2 writes across the ring's end: its last 95 words go to the mirror,
+// where step 3 reads them, and to the start.
+//
+// Bound: shared memory and the step's own latency.  A value takes seven 4-byte accesses (four
+// ring words, two tables, one store) and one global store, 8 of the SM's memory cycles per 32
+// values: 66.7 us for 2^26 values on an SM with four of the 512 generators; the rest is the
+// chain of a step (load, table, store, barrier), which four blocks overlap only in part.  With
+// the offsets wrapped by masks at run time, each step was 36 instructions a value.  2^26 values
+// on one B200, before -> now: uniform fp32 112.7 -> 100.4 us, uniform fp64 274 -> 198, normal
+// fp32 (packed transform either way) 165 -> 153, fp64 468 either way, Poisson 168 -> 133.
 template<class F>
 __global__ void __launch_bounds__(kMtgpBlock, 4) mtgp_fill(MtgpArgs a, F fw)
 {
-    __shared__ uint32_t        s[kMtgpState];
+    // 4 blocks of 256 threads per SM (at most 64 registers): all 512 block generators resident
+    // at once on 148 SMs
+    __shared__ uint32_t        s[kMtgpState + kMtgpMirror];
     __shared__ uint32_t        tbl[16], tmp[16];
     extern __shared__ unsigned char smem[];
     const F                    f = stage_table(fw, smem);
     const uint32_t             b = blockIdx.x, t = threadIdx.x;
     const uint32_t*            p = a.params + b * kMtgpWords;
-    for(int i = t; i < kMtgpState; i += kMtgpBlock)
-        s[i] = a.rings[b * kMtgpState + i];
+    const int                  k = a.offsets[b];
+    for(int i = static_cast<int>(t); i < kMtgpState; i += kMtgpBlock)
+        s[i] = a.rings[b * kMtgpState + ((k + i) & kMtgpMask)];
     if(t < 16)
     {
         tbl[t] = p[3 + t];
@@ -82,63 +101,94 @@ __global__ void __launch_bounds__(kMtgpBlock, 4) mtgp_fill(MtgpArgs a, F fw)
     }
     const int      pos = static_cast<int>(p[0]);
     const uint32_t sh1 = p[1], sh2 = p[2], mask = p[35];
-    int            k   = a.offsets[b];
+    uint32_t*      at  = s + t;           // this thread's word of the step at offset 0
+    uint32_t*      far = s + t + pos - 1; // and its pos - 1 (tempering) and pos words
     __syncthreads();
 
-    // one block step: this thread's value, then every thread's writes become visible
-    auto step = [&]() -> uint32_t {
-        uint32_t x = (s[(k + t) & kMtgpMask] & mask) ^ s[(k + t + 1) & kMtgpMask];
-        uint32_t y = s[(k + t + pos) & kMtgpMask];
-        x ^= x << sh1;
-        y                                 = x ^ (y >> sh2);
-        const uint32_t r                  = y ^ tbl[y & 0x0f];
-        s[(k + t + kMtgpN) & kMtgpMask]   = r;
-        uint32_t tt                       = s[(k + t + pos - 1) & kMtgpMask];
+    // entry (v & 15) of a 16-word table
+    auto entry = [](const uint32_t* table, uint32_t v) {
+        return *reinterpret_cast<const uint32_t*>(reinterpret_cast<const unsigned char*>(table) + ((v << 2) & 60u));
+    };
+    // one block step at ring offset 256 ph: this thread's value, then every thread's writes
+    // become visible
+    auto step = [&](int ph) -> uint32_t {
+        const int o  = static_cast<int>(kMtgpBlock) * ph;
+        uint32_t  x  = (at[o] & mask) ^ at[o + 1];
+        uint32_t  tt = far[o];
+        uint32_t  y  = far[o + 1];
+        y            = x ^ (x << sh1) ^ (y >> sh2);
+        const uint32_t r = y ^ entry(tbl, y);
+        if(ph == 2)
+        {
+            at[o + kMtgpN] = r; // the last 95 threads': words of the mirror
+            if(t >= kMtgpState - (2 * kMtgpBlock + kMtgpN))
+                at[o + kMtgpN - kMtgpState] = r;
+        }
+        else
+        {
+            at[ph == 3 ? o + kMtgpN - kMtgpState : o + kMtgpN] = r;
+        }
         tt ^= tt >> 16;
         tt ^= tt >> 8;
         __syncthreads();
-        k = (k + kMtgpBlock) & kMtgpMask;
-        return r ^ tmp[tt & 0x0f];
+        return r ^ entry(tmp, tt);
     };
 
     using T                      = typename F::T;
     constexpr unsigned ow        = F::ow;
     constexpr unsigned VB        = ow * sizeof(T);
-    const unsigned long long str = static_cast<unsigned long long>(kMtgpGens) * kMtgpBlock;
+    constexpr unsigned long long str = static_cast<unsigned long long>(kMtgpGens) * kMtgpBlock;
     unsigned long long index     = static_cast<unsigned long long>(b) * kMtgpBlock + t;
-    uint32_t           in[F::iw];
-    T                  out[ow];
-    auto               gen = [&]() {
-#pragma unroll
-        for(unsigned i = 0; i < F::iw; i++)
-            in[i] = step();
-        f(in, out);
-    };
+    constexpr unsigned U         = kMtgpUnits<F>;
+    static_assert(U * F::iw % 4 == 0, "whole turns");
     // index < vec_n_down and index < vec_n_up are the same in the whole block (both are
     // multiples of 256), so every thread takes every step
-    if constexpr(long_transform<F>::value)
+    unsigned char* dst = a.vec + index * VB;
+    for(; index + (U - 1) * str < a.vec_n_down; index += U * str, dst += U * str * VB)
     {
-        // U rounds' steps, then their transforms with no branch between them: the U
-        // Box-Muller chains interleave instead of each waiting out its own latency
-        constexpr unsigned U = kMtgpUnits<F>;
-        while(index + (U - 1) * str < a.vec_n_down)
+        uint32_t in[U][F::iw];
+        T        o[U][ow];
+        // a long transform after all steps, with no branch between its units, so that their
+        // chains interleave instead of each waiting out its own latency
+#pragma unroll
+        for(unsigned u = 0; u < U; u++)
         {
-            uint32_t in[U][F::iw];
 #pragma unroll
-            for(unsigned u = 0; u < U; u++)
-#pragma unroll
-                for(unsigned i = 0; i < F::iw; i++)
-                    in[u][i] = step();
-            T o[U][ow];
+            for(unsigned i = 0; i < F::iw; i++)
+                in[u][i] = step((u * F::iw + i) % 4);
+            if constexpr(!long_transform<F>::value)
+            {
+                f(in[u], o[u]);
+                store_small(dst + u * str * VB, o[u]);
+            }
+        }
+        if constexpr(long_transform<F>::value)
+        {
 #pragma unroll
             for(unsigned u = 0; u < U; u += 2)
                 apply_pair(f, in[u], in[u + 1], o[u], o[u + 1]);
 #pragma unroll
             for(unsigned u = 0; u < U; u++)
-                store_small(a.vec + (index + u * str) * VB, o[u]);
-            index += U * str;
+                store_small(dst + u * str * VB, o[u]);
         }
     }
+    // the rest of the rounds, the round that is not whole, and the head and tail: a step's
+    // offset at run time, the next turn's first step on
+    uint32_t in[F::iw];
+    T        out[ow];
+    int      ph  = 0;
+    auto     gen = [&]() {
+#pragma unroll 1
+        for(unsigned i = 0; i < F::iw; i++)
+        {
+            const uint32_t v = step(ph);
+            ph               = (ph + 1) & 3;
+#pragma unroll
+            for(unsigned j = 0; j < F::iw; j++)
+                in[j] = i == j ? v : in[j];
+        }
+        f(in, out);
+    };
     while(index < a.vec_n_down)
     {
         gen();
@@ -163,10 +213,11 @@ __global__ void __launch_bounds__(kMtgpBlock, 4) mtgp_fill(MtgpArgs a, F fw)
             for(unsigned o = 0; o < a.tail; o++)
                 data[a.n - a.tail + o] = out[o];
     }
-    for(int i = t; i < kMtgpState; i += kMtgpBlock)
-        a.rings[b * kMtgpState + i] = s[i];
+    // whole turns leave the offset where it was
+    for(int i = static_cast<int>(t); i < kMtgpState; i += kMtgpBlock)
+        a.rings[b * kMtgpState + ((k + i) & kMtgpMask)] = s[i];
     if(t == 0)
-        a.offsets[b] = k;
+        a.offsets[b] = (k + static_cast<int>(kMtgpBlock) * ph) & kMtgpMask;
 }
 
 // mtgp_fill on the host (CPU path of the host generators): generator b's 256 threads take
