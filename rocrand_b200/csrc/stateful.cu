@@ -171,13 +171,20 @@ struct FillArgs
     unsigned long long n, vec_n;
 };
 
+// Threads per block of the fill.  The E = 131072 slots are 1024 blocks of 128, 6.92 per SM, so
+// the fullest SM holds 7 and the others as many or one fewer; as 512 blocks of 256 they were
+// 3.46, and the SMs with 4 worked on while the others had run out.  2^26 values a call on one
+// B200, 256 -> 128 threads: XORWOW normal fp32 85.3 -> 77.5 us, fp64 270 -> 242, uint (bound by
+// HBM) 51.3 -> 49.6; MRG32k3a uint 132.7 -> 118.3; LFSR113 uint 73.5 -> 64.6.
+constexpr unsigned kFillBlock = 128;
+
 template<class E, class F>
-__global__ void __launch_bounds__(kBlock) stateful_fill(FillArgs a, F f)
+__global__ void __launch_bounds__(kFillBlock) stateful_fill(FillArgs a, F f)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const F g = stage_table(f, smem);
 
-    const uint32_t t = blockIdx.x * kBlock + threadIdx.x; // slot
+    const uint32_t t = blockIdx.x * kFillBlock + threadIdx.x; // slot
     if(t >= kE)
         return;
     const bool loops = t < a.vec_n;
@@ -958,7 +965,10 @@ private:
         else if(n > 0)
         {
             const size_t smem = table_smem_bytes(f);
-            stateful_fill<Eng, F><<<kE / kBlock, kBlock, smem, m_stream>>>(a, f);
+            // the slots that write: vector j's is j mod E, and the edges' follows the last vector
+            const unsigned long long slots = std::min<unsigned long long>(a.vec_n + 1, kE);
+            const unsigned           grid  = static_cast<unsigned>((slots + kFillBlock - 1) / kFillBlock);
+            stateful_fill<Eng, F><<<grid, kFillBlock, smem, m_stream>>>(a, f);
             const rocrand_status st = launch_status();
             if(st != ROCRAND_STATUS_SUCCESS)
                 return st;
