@@ -70,30 +70,29 @@ struct Mrg32k3aEngine // rocrand_mrg32k3a.h:160-190: g1[0..2], g2[0..2]
     static constexpr int      kUnroll = 6; // two rotation periods of the three-word components
     static constexpr uint64_t kM1 = 4294967087ull, kM2 = 4294944443ull;
     uint32_t                  w[kWords];
-    // t < 2 m: t mod m, with the comparison and subtraction on 32-bit words (t - m < 2^32)
-    __host__ __device__ __forceinline__ static uint32_t sub_once(uint64_t t, uint32_t m)
+    // x mod m for m = 2^32 - c and 2^32 hi + lo = x + 2^32, x = c (hi - 1) + lo (mod m) < 2 m:
+    // with u = c hi + lo = that + c, the sum reaches m just when u reaches 2^32, where its low
+    // word is the remainder; below, u - c is.  (2^26 uint on one B200, against comparing the
+    // folded sum with m in 64 bits: 118.3 -> 99.4 us; bound by the wide products, four cycles
+    // of a scheduler each, and issue.)
+    __host__ __device__ __forceinline__ static uint32_t fold(uint64_t x_plus, uint32_t c)
     {
-        const uint32_t lo = static_cast<uint32_t>(t);
-        return (static_cast<uint32_t>(t >> 32) != 0u || lo >= m) ? lo - m : lo;
-    }
-    // p < 2^54: 2^32 = 209 (mod m1) folds p below 2^33 < 2 m1
-    __host__ __device__ __forceinline__ static uint32_t mod_m1(uint64_t p)
-    {
-        return sub_once(209ull * (p >> 32) + (p & 0xffffffffull), static_cast<uint32_t>(kM1));
-    }
-    // p < 2^54: two folds by 2^32 = 22853 (mod m2) bring p below 2^33 < 2 m2
-    __host__ __device__ __forceinline__ static uint32_t mod_m2(uint64_t p)
-    {
-        p = 22853ull * (p >> 32) + (p & 0xffffffffull);
-        return sub_once(22853ull * (p >> 32) + (p & 0xffffffffull), static_cast<uint32_t>(kM2));
+        const uint32_t lo = static_cast<uint32_t>(x_plus);
+        const uint32_t u  = c * static_cast<uint32_t>(x_plus >> 32) + lo;
+        return u - (u >= lo ? c : 0u);
     }
     __host__ __device__ __forceinline__ uint32_t next()
     {
-        const uint32_t p1 = mod_m1(1403580ull * w[1] + 810728ull * static_cast<uint32_t>(static_cast<uint32_t>(kM1) - w[0]));
+        // a product sum is below 2^54; modulo m1 one fold by 2^32 = 209 leaves it below 2^33,
+        // modulo m2 the first of two folds by 22853 leaves it below 2^37
+        const uint32_t n1 = static_cast<uint32_t>(kM1) - w[0];
+        const uint32_t p1 = fold((1ull << 32) + 1403580ull * w[1] + 810728ull * n1, 209u);
         w[0] = w[1];
         w[1] = w[2];
         w[2] = p1;
-        const uint32_t p2 = mod_m2(527612ull * w[5] + 1370589ull * static_cast<uint32_t>(static_cast<uint32_t>(kM2) - w[3]));
+        const uint32_t n2 = static_cast<uint32_t>(kM2) - w[3];
+        const uint64_t q  = 527612ull * w[5] + 1370589ull * n2;
+        const uint32_t p2 = fold((1ull << 32) + static_cast<uint32_t>(q) + 22853ull * static_cast<uint32_t>(q >> 32), 22853u);
         w[3] = w[4];
         w[4] = w[5];
         w[5] = p2;
