@@ -9,22 +9,23 @@
 // logf (glibc) is not correctly rounded: on the ~11.6 million distinct arguments this
 // formula can produce, 0.93 % of its results are the other neighbour of the exact value.
 //
-// Method.  The kernels evaluate the logarithm L = hi + lo as a pair of floats to about 2^-44
-// relative (base(): a table-driven reduction in single precision whose first sums are exact)
-// and take f = hi, its rounding to float.  A host result that differs from f can only be f's
-// other neighbour on L's side of f (the host's error is below one ulp), and only where L lies
-// close to the midpoint between the two.  The build (rocrand_b200/data/make_logf_replay.cpp)
-// runs the host's logf over every argument the formula can reach and records
+// Method.  The kernels evaluate the logarithm L = hi + lo as a pair of floats (base(): a
+// table-driven reduction in single precision; at worst 2^-7.6 of an ulp off, 2^-11 below 0.9) and take f = hi, its rounding to float.  A host result that differs
+// from f can only be f's other neighbour on L's side of f (the host's error is below one ulp),
+// and only where L lies close to the midpoint between the two.  The build
+// (rocrand_b200/data/make_logf_replay.cpp) runs the host's logf over every argument the formula
+// can reach and records
 //  * per bucket of arguments (the float's bits >> kBucketShift) and side of f (L below f, L
-//    above f), the largest distance of L from the midpoint, in units of 2^-16 ulp (plus one),
-//    of an argument whose host result differs from f (0: none);
+//    above f), the smallest |lo| / 2^exponent(hi) of an argument whose host result differs from
+//    f, as the upper 16 bits of a float, rounded down (none: infinity);
 //  * those arguments, as a set: a bucketed two-choice hash table of 32-bit keys, four per
 //    16-byte bucket, so a lookup is two independent 16-byte loads.
-// An argument within its bucket's bound for its side tests membership (about 1 % of
+// An argument that reaches its bucket's threshold for its side tests membership (about 1.5 % of
 // arguments), and a member returns f's neighbour on L's side; all others return f.  The build
 // then replays every reachable argument through this same code on the host and requires the
-// host's logf result for each.  base() is IEEE float operations only and the distance and
-// lookup integer ones, so the host and device builds of this header agree bit for bit.
+// host's logf result for each, which is also what makes base()'s accuracy enough.  base() and
+// the test are IEEE float operations and the lookup integer ones, so the host and device builds
+// of this header agree bit for bit.
 #pragma once
 
 #include "ieee.cuh"
@@ -46,7 +47,7 @@ constexpr uint32_t kHash2       = 0x85EBCA77u;
 // The tables as the kernels see them (device pointers).
 struct Table
 {
-    const uint32_t* bound        = nullptr; // kBuckets entries: side 0 in bits 0-15, side 1 in 16-31
+    const uint32_t* bound        = nullptr; // kBuckets thresholds: side 0 in bits 0-15, side 1 in 16-31
     const uint4*    keys         = nullptr; // buckets of four member arguments; 0 = empty slot
     uint32_t        log2_buckets = 0;
 };
@@ -90,15 +91,12 @@ RB_PM_HD T ld(const T* p)
 #endif
 }
 
-// f = the float rounding of log(t) for t in [2^-64, 1], the side of f on which the logarithm
-// lies (1: above) and its distance from the midpoint between f and its neighbour on that
-// side, in units of 2^-16 ulp of f (0 .. 32768; larger = safer; within one unit).
+// f = the float rounding of log(t) for t in [2^-25, 1], and what L has beyond it.
 //   t = 2^k z, z in [OFF, 2 OFF) by integer operations; r = z invc - 1 exact (|r| < 2^-7,
-//   invc with at most 8 significant bits); log t = (k ln2_hi + head) + r - r^2/2
-//   + r^3 (1/3 - r/4 + r^2/5 - r^3/6) + (tail + k ln2_lo): the first sum exact, the next two
-//   compensated (two-sum, exact square), the rest in plain float; r^7/7 is below 2^-44 of
-//   the result.
-RB_PM_HD float base(float t, uint32_t& dist, uint32_t& side)
+//   invc with at most 8 significant bits); log t = (k ln2_hi + head) + r + w + (tail + k
+//   ln2_lo) with w = r^2 (-1/2 + r/3 - r^2/4 + r^3/5): the first term is exact, r + w and the
+//   sum with it are compensated (|first term| >= |r| or it is 0), the rest plain float.
+RB_PM_HD float base(float t, float& lo)
 {
     const uint32_t ix  = fbits(t);
     const uint32_t tmp = ix - RB_LOGF_OFF;
@@ -109,52 +107,44 @@ RB_PM_HD float base(float t, uint32_t& dist, uint32_t& side)
     const float    kf  = static_cast<float>(k);
     const float    r   = ieee::ffma(z, row.x, -1.0f);          // exact
     const float    a   = ieee::ffma(kf, RB_LN2F_HI, row.y);    // exact: multiples of 2^-19, |a| < 2^5
-    // s1 + e1 = a + r exactly (two-sum)
-    const float s1 = ieee::fadd(a, r);
-    const float bb = ieee::fsub(s1, a);
-    const float e1 = ieee::fadd(ieee::fsub(a, ieee::fsub(s1, bb)), ieee::fsub(r, bb));
-    // -r^2 / 2 = q + ql exactly
-    const float r2 = ieee::fmul(r, r);
-    const float q  = ieee::fmul(-0.5f, r2);
-    const float ql = ieee::fmul(-0.5f, ieee::ffma(r, r, -r2));
-    // s2 + e2 = s1 + q exactly: |s1| >= |q| (s1 = r when a = 0, else |s1| > 2^-9)
-    const float s2 = ieee::fadd(s1, q);
-    const float e2 = ieee::fsub(q, ieee::fsub(s2, s1));
-    float       p  = ieee::ffma(-1.0f / 6.0f, r, 1.0f / 5.0f);
-    p              = ieee::ffma(p, r, -1.0f / 4.0f);
-    p              = ieee::ffma(p, r, 1.0f / 3.0f);
-    const float tail = ieee::fmul(p, ieee::fmul(r2, r));
-    const float low  = ieee::fadd(ieee::fadd(ieee::fadd(e1, e2), ieee::fadd(ql, row.z)),
-                                  ieee::ffma(kf, RB_LN2F_LO, tail));
-    const float hi = ieee::fadd(s2, low);
-    const float lo = ieee::fsub(low, ieee::fsub(hi, s2)); // |lo| <= ulp(hi) / 2
-    // |lo| in units of 2^-16 ulp of hi, by a power-of-two scale (exact), and the distance of
-    // L from the midpoint half an ulp away.  (Where |hi| is a power of two and lo points
-    // inward the midpoint is a quarter of an ulp away; the distance only has to order the
-    // arguments, and the build's bounds are taken in this same measure.)
-    uint32_t e = (fbits(hi) >> 23) & 0xffu;
-    e          = e < 39u ? 39u : e; // hi = 0 (t = 1): lo = 0 too
-    const float y = ieee::fmul(fabsf(lo), ffrom((293u - e) << 23)); // |lo| 2^(166 - e)
-    dist          = 32768u - static_cast<uint32_t>(y);
-    side          = lo > 0.0f ? 1u : 0u;
+    float          p   = ieee::ffma(1.0f / 5.0f, r, -1.0f / 4.0f);
+    p                  = ieee::ffma(p, r, 1.0f / 3.0f);
+    p                  = ieee::ffma(p, r, -0.5f);
+    const float w      = ieee::fmul(p, ieee::fmul(r, r));
+    const float c      = ieee::fadd(r, w);
+    const float cl     = ieee::fsub(w, ieee::fsub(c, r));
+    const float s      = ieee::fadd(a, c);
+    const float sl     = ieee::fsub(c, ieee::fsub(s, a));
+    const float low    = ieee::fadd(ieee::fadd(sl, cl), ieee::ffma(kf, RB_LN2F_LO, row.z));
+    const float hi     = ieee::fadd(s, low);
+    lo                 = ieee::fsub(low, ieee::fsub(hi, s)); // |lo| <= ulp(hi) / 2
     return hi;
+}
+
+// 2^exponent of f (0 for f = 0): what the thresholds are relative to.
+RB_PM_HD float exponent_of(float f)
+{
+    return ffrom(fbits(f) & 0x7f800000u);
+}
+
+// The threshold of lo's side in a bucket's word.
+RB_PM_HD float threshold_of(uint32_t word, float lo)
+{
+    return ffrom(lo > 0.0f ? word & 0xffff0000u : word << 16);
 }
 
 // Key buckets of argument `key` in a table of 2^lb buckets.
 RB_PM_HD uint32_t bucket1(uint32_t key, uint32_t lb) { return (key * kHash1) >> (32 - lb); }
 RB_PM_HD uint32_t bucket2(uint32_t key, uint32_t lb) { return (key * kHash2) >> (32 - lb); }
 
-// The host C library's logf(t) for an argument of the inverse-erf normal.
+// The host C library's logf(t) for an argument of the inverse-erf normal, t >= 2^-24 or so (t = 0
+// gives some number).
 RB_PM_HD float logf_host(float t, const Table& tb)
 {
-    if(!(t >= 0x1p-64f) || !(t <= 1.0f))
-        return pm::logf(t); // zero (-inf) and anything outside the formula's range
-    uint32_t    dist, side;
-    const float    f     = base(t, dist, side);
-    const uint32_t key   = fbits(t);
-    const uint32_t b2    = ld(tb.bound + (key >> kBucketShift));
-    const uint32_t bound = side ? (b2 >> 16) : (b2 & 0xffffu);
-    if(dist >= bound)
+    float          lo;
+    const float    f   = base(t, lo);
+    const uint32_t key = fbits(t);
+    if(!(fabsf(lo) >= ieee::fmul(threshold_of(ld(tb.bound + (key >> kBucketShift)), lo), exponent_of(f))))
         return f;
     const uint4 a   = ld(tb.keys + bucket1(key, tb.log2_buckets));
     const uint4 b   = ld(tb.keys + bucket2(key, tb.log2_buckets));
@@ -165,7 +155,7 @@ RB_PM_HD float logf_host(float t, const Table& tb)
     // f's neighbour on L's side: one step of the bit pattern, away from zero when L lies
     // beyond f in f's direction
     const uint32_t fb = fbits(f);
-    return ffrom((side != 0u) == ((fb >> 31) == 0u) ? fb + 1u : fb - 1u);
+    return ffrom((lo > 0.0f) == ((fb >> 31) == 0u) ? fb + 1u : fb - 1u);
 }
 
 } // namespace lr

@@ -75,8 +75,35 @@ inline unsigned long long sobol_chunk(unsigned long long n, unsigned long long d
     return best_chunk;
 }
 
+// Points per block of the 8-byte kinds that only store: 32 KiB of output, less where that
+// leaves blocks out of the first wave.  Many short blocks in the order of memory keep the writes
+// of the moment together: plain stores of 1 GiB run at 7.2-7.4 TB/s in blocks of 28 to 112 KiB
+// and at 6.0-6.3 TB/s in one wave of long runs or grid strides, whose blocks drift apart.  64
+// dimensions, 2^26 uniform fp64 on one B200, by whole waves -> by 32 KiB: Sobol32 150 -> 137 us,
+// scrambled Sobol64 157 -> 116 (2^24: 62.8 -> 34.6).  The 4-byte kinds gain nothing or lose
+// (uniform fp32 44.6 -> 49.3: a block's start costs them more) and keep whole waves.
+inline unsigned long long sobol_store_chunk(unsigned long long n, unsigned long long dims,
+                                            unsigned long long group, unsigned long long wave, size_t size)
+{
+    const unsigned long long full   = 32768 / (group * size);
+    const unsigned long long spread = (n + group - 1) / group * dims / (wave == 0 ? 1 : wave);
+    const unsigned long long per    = std::max<unsigned long long>(1, std::min(full, spread));
+    return per * group;
+}
+
+// Blocks that an SM has to hold: all eight for the kinds that are little more than a store (with
+// seven, 64 dimensions x 2^20 uint32 were cut into 16 long runs a row, 1024 streams of one wave,
+// and took 86 us instead of 45 on one B200); the transforms may use the registers for the four
+// points they work on side by side.
+template<SobolKind K>
+constexpr unsigned kSobolBlocks = K == SobolKind::UINT || K == SobolKind::ULL || K == SobolKind::UCHAR
+                                          || K == SobolKind::USHORT || K == SobolKind::FLOAT
+                                          || K == SobolKind::DOUBLE || K == SobolKind::HALF
+                                      ? 8u
+                                      : 1u;
+
 template<class W, SobolKind K>
-__global__ void __launch_bounds__(kBlock) sobol_fill(SobolCall<W> a)
+__global__ void __launch_bounds__(kBlock, kSobolBlocks<K>) sobol_fill(SobolCall<W> a)
 {
     using T                = typename SobolOut<K, W>::T;
     constexpr int      B   = 8 * sizeof(W);
@@ -124,17 +151,38 @@ __global__ void __launch_bounds__(kBlock) sobol_fill(SobolCall<W> a)
             if((g >> b) & 1)
                 x ^= v[b];
     }
+    // Point i to i + 1 flips the direction vector of i's lowest zero bit: number 0, 1, 0 after
+    // i = 0, 1, 2 (mod 4), and one to look up after i = 3 (mod 4).  A thread's points start at the
+    // same residue every time (strides are multiples of 4), so of four steps three have their
+    // vector in a register.  (The 32-bit kinds that only store look every one up: their kernel
+    // waits for memory, and 2^26 uniform fp32 is 45 us that way and 48 this.)
+    constexpr bool kLookAll = sizeof(W) == 4 && kSobolBlocks<K> > 1;
+    const unsigned residue  = static_cast<unsigned>(i) & 3u;
+    const W        v0 = v[0], v1 = v[1], vl = v[lg - 1];
     for(; p < end; p += stride)
     {
         T out[PPT];
+        W look[PPT / 4];
+        if constexpr(!kLookAll)
+        {
+#pragma unroll
+            for(unsigned j = 0; j < PPT / 4; j++)
+                look[j] = v[rzb(static_cast<I>((i + 4 * j) | 3u))];
+        }
         W xx = x;
-        I ii = i;
 #pragma unroll
         for(unsigned k = 0; k < PPT; k++)
         {
             out[k] = sobol_apply<K, W>(xx ^ c, a.p, cdf);
-            xx ^= v[rzb(ii)];
-            ii++;
+            if constexpr(kLookAll)
+            {
+                xx ^= v[rzb(static_cast<I>(i + k))];
+            }
+            else
+            {
+                const unsigned at = (residue + k) & 3u;
+                xx ^= at == 3u ? look[k / 4] : (at == 1u ? v1 : v0);
+            }
         }
         if(vec_ok && p + PPT <= a.n)
         {
@@ -161,7 +209,7 @@ __global__ void __launch_bounds__(kBlock) sobol_fill(SobolCall<W> a)
         }
         // leap-frog by the power-of-two stride 2^lg: Gray-code bit lg-1 flips, and the bit of
         // the lowest zero of i above the low lg bits (rocrand_sobol32.h:140-159)
-        x ^= v[lg - 1];
+        x ^= vl;
         x ^= v[rzb(static_cast<I>(i | static_cast<I>(stride - 1)))];
         i += static_cast<I>(stride);
     }
@@ -351,7 +399,9 @@ private:
         {
             const unsigned long long wave
                 = static_cast<unsigned long long>(device_info().sm_count) * blocks_per_sm(kernel, smem);
-            m_chunk        = sobol_chunk(N, m_dims, group, wave);
+            m_chunk        = K == SobolKind::DOUBLE || K == SobolKind::ULL
+                                 ? sobol_store_chunk(N, m_dims, group, wave, sizeof(T))
+                                 : sobol_chunk(N, m_dims, group, wave);
             m_chunk_kernel = kernel;
             m_chunk_n      = N;
             m_chunk_smem   = smem;

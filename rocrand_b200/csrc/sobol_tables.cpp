@@ -148,7 +148,7 @@ bool logf_replay_device(lr::Table& out)
         const unsigned char* blob  = rb200_logf_replay_begin;
         const size_t         bytes = static_cast<size_t>(rb200_logf_replay_end - rb200_logf_replay_begin);
         uint32_t             h[6];
-        if(bytes < 32 || std::memcmp(blob, "RBLOGF02", 8) != 0)
+        if(bytes < 32 || std::memcmp(blob, "RBLOGF03", 8) != 0)
             return false;
         std::memcpy(h, blob + 8, sizeof(h));
         const size_t bound_bytes = static_cast<size_t>(h[1]) * 4;

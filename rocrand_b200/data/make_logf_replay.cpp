@@ -11,15 +11,16 @@
 // 2. For each distinct t, the host's logf(t) against the kernels' float f of the logarithm
 //    (logf_replay.cuh base(), compiled here for the host: the same IEEE operations).  Where
 //    they differ, the host's result must be f's neighbour on the logarithm's side of f; the
-//    argument joins the member set, and the bound of its bucket and side is raised to its
-//    distance from the midpoint plus one.
+//    argument joins the member set, and the threshold of its bucket and side is lowered to its
+//    |lo| / 2^exponent(f), rounded down to the upper 16 bits of a float.
 // 3. The member set goes into a bucketed two-choice hash table (four keys per bucket, cuckoo
 //    insertion; the table doubles until every key has a place).
 // 4. Every t is replayed through logf_replay.cuh logf_host() with the finished tables and
-//    must give the host's logf(t) bit for bit; otherwise nothing is written.
+//    must give the host's logf(t) bit for bit; otherwise nothing is written.  (t = 0, which the
+//    normal treats by itself, is not replayed.)
 //
-// Output (little-endian): "RBLOGF02", u32 bucket shift, u32 bucket count, u32 log2 of the
-// key-bucket count, u32 members, u32 reachable arguments, u32 0; u32 bounds [bucket count]
+// Output (little-endian): "RBLOGF03", u32 bucket shift, u32 bucket count, u32 log2 of the
+// key-bucket count, u32 members, u32 reachable arguments, u32 0; u32 thresholds [bucket count]
 // (side 0 in the low half, side 1 in the high half) padded to 16 bytes; u32 keys [4 x key
 // buckets].
 #include "logf_replay.cuh"
@@ -104,52 +105,53 @@ int main(int argc, char** argv)
     seen.shrink_to_fit();
 
     // 2. differences between the host's logf and the kernels' rounding
+    args.erase(std::remove(args.begin(), args.end(), 0u), args.end());
     const size_t          na = args.size();
-    std::vector<uint32_t> host(na), dist(na, 0), side(na, 0);
+    std::vector<uint32_t> host(na);
     std::vector<uint8_t>  state(na, 0); // 0 same, 1 member, 2 not in range, 3 not the neighbour
 #pragma omp parallel for schedule(dynamic, 4096)
     for(long long i = 0; i < static_cast<long long>(na); i++)
     {
         const float t = lr::ffrom(args[i]);
         host[i]       = lr::fbits(::logf(t));
-        if(!(t >= 0x1p-64f) || !(t <= 1.0f))
+        if(!(t >= 0x1p-25f) || !(t <= 1.0f))
         {
-            state[i] = lr::fbits(pm::logf(t)) != host[i] ? 2 : 0;
+            state[i] = 2;
             continue;
         }
-        uint32_t    d, s;
-        const float f = lr::base(t, d, s);
-        dist[i]       = d;
-        side[i]       = s;
+        float       lo;
+        const float f = lr::base(t, lo);
         if(lr::fbits(f) == host[i])
             continue;
         const uint32_t fb = lr::fbits(f);
-        const uint32_t nb = (s != 0u) == ((fb >> 31) == 0u) ? fb + 1u : fb - 1u;
+        const uint32_t nb = (lo > 0.0f) == ((fb >> 31) == 0u) ? fb + 1u : fb - 1u;
         state[i]          = nb == host[i] ? 1 : 3;
     }
-    std::vector<uint32_t> bound(lr::kBuckets, 0);
+    std::vector<uint32_t> bound(lr::kBuckets, 0x7f807f80u); // no member: infinity
     std::vector<uint32_t> members;
     for(size_t i = 0; i < na; i++)
     {
         if(state[i] >= 2)
         {
             std::fprintf(stderr, "argument %08x: %s\n", args[i],
-                         state[i] == 2 ? "outside [2^-64, 1] differs from the host"
+                         state[i] == 2 ? "outside [2^-25, 1]"
                                        : "the host's result is not the neighbour on the logarithm's side");
             return 1;
         }
         if(state[i] == 0)
             continue;
+        float          lo;
+        const float    f   = lr::base(lr::ffrom(args[i]), lo);
         const uint32_t key = args[i] >> lr::kBucketShift;
-        const uint32_t b   = dist[i] + 1u;
-        if(key >= lr::kBuckets || b > 65535u)
+        if(key >= lr::kBuckets || f == 0.0f)
         {
-            std::fprintf(stderr, "argument %08x: bucket %u, bound %u out of range\n", args[i], key, b);
+            std::fprintf(stderr, "argument %08x: bucket %u, logarithm %g\n", args[i], key, f);
             return 1;
         }
-        const uint32_t sh  = side[i] ? 16 : 0;
+        const uint32_t b   = lr::fbits(std::fabs(lo) / lr::exponent_of(f)) >> 16; // exact quotient, cut down
+        const uint32_t sh  = lo > 0.0f ? 16 : 0;
         const uint32_t cur = (bound[key] >> sh) & 0xffffu;
-        if(b > cur)
+        if(b < cur)
             bound[key] = (bound[key] & ~(0xffffu << sh)) | (b << sh);
         members.push_back(args[i]);
     }
@@ -174,11 +176,9 @@ int main(int argc, char** argv)
         const float t = lr::ffrom(args[i]);
         if(lr::fbits(lr::logf_host(t, tb)) != host[i])
             bad++;
-        if(t >= 0x1p-64f && t <= 1.0f)
-        {
-            const uint32_t b = (bound[args[i] >> lr::kBucketShift] >> (side[i] ? 16 : 0)) & 0xffffu;
-            probed += dist[i] < b ? 1 : 0;
-        }
+        float       lo;
+        const float f = lr::base(t, lo);
+        probed += std::fabs(lo) >= lr::threshold_of(bound[args[i] >> lr::kBucketShift], lo) * lr::exponent_of(f) ? 1 : 0;
     }
     std::printf("logf replay: %zu reachable arguments, %zu differ from the kernels' rounding "
                 "(%.3f%%), %.2f%% looked up, %u key buckets, %lld mismatches\n",
@@ -191,7 +191,7 @@ int main(int argc, char** argv)
         return 1;
     const uint32_t hdr[6] = {static_cast<uint32_t>(lr::kBucketShift), lr::kBuckets, lb,
                              static_cast<uint32_t>(members.size()), static_cast<uint32_t>(na), 0u};
-    std::fwrite("RBLOGF02", 1, 8, f);
+    std::fwrite("RBLOGF03", 1, 8, f);
     std::fwrite(hdr, 4, 6, f);
     std::fwrite(bound.data(), 4, bound.size(), f);
     const size_t pad      = (16 - (8 + 24 + 4 * bound.size()) % 16) % 16;
