@@ -73,13 +73,14 @@ inline int blocks_per_sm(const void* fn, size_t smem)
 }
 
 // Grid for a grid-stride kernel over `work` items: enough resident blocks to fill every
-// SM, never more than the work needs.
+// SM (less `reserved` that the caller adds), never more than the work needs.
 template<class Kernel>
-inline unsigned grid_for(Kernel k, unsigned long long work, size_t smem)
+inline unsigned grid_for(Kernel k, unsigned long long work, size_t smem, unsigned reserved = 0)
 {
     const int                per  = blocks_per_sm(reinterpret_cast<const void*>(k), smem);
     const unsigned long long full = static_cast<unsigned long long>(device_info().sm_count)
-                                    * static_cast<unsigned long long>(per);
+                                        * static_cast<unsigned long long>(per)
+                                    - reserved;
     const unsigned long long need = (work + kBlock - 1) / kBlock;
     unsigned long long       g    = need < full ? need : full;
     return static_cast<unsigned>(g < 1 ? 1 : g);

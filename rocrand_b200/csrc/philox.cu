@@ -29,6 +29,33 @@
 namespace rb200
 {
 
+// A call with a head or tail has one block more, which makes them alone: a unit to a thread,
+// the head's in the first warp and the tail's in the second.  (As one thread's sequential runs
+// behind block 0's vectors they were up to 1.5 us of every such call.)
+template<class F>
+__device__ __forceinline__ bool philox_edges(const PhiloxCall& a, const F& g)
+{
+    if(a.head + a.tail == 0 || blockIdx.x + 1 != gridDim.x)
+        return false;
+    using T                        = typename F::T;
+    const bool               tail  = threadIdx.x >= 32;
+    const uint32_t           unit  = threadIdx.x & 31u;
+    const uint32_t           count = threadIdx.x >= 64 ? 0u : (tail ? a.tail : a.head);
+    const unsigned long long pos
+        = tail ? 4 * a.vec_n + ((a.vec_n % kPhiloxRefStride) == 0 ? a.start0 : a.head) : 0ull;
+    T* out = reinterpret_cast<T*>(a.data) + (tail ? a.n - a.tail : 0ull);
+    if(unit * F::ow < count)
+        philox_scalar_run(a, g, pos + unit * F::iw, out + unit * F::ow,
+                          count - unit * F::ow < F::ow ? count - unit * F::ow : F::ow);
+    return true;
+}
+
+// Blocks that take vectors.
+__device__ __forceinline__ uint32_t philox_blocks(const PhiloxCall& a)
+{
+    return gridDim.x - (a.head + a.tail == 0 ? 0u : 1u);
+}
+
 // kAligned: start0 == head and (s0 + head) % 4 == 0, so vector j is exactly block
 // c0 + (s0 + head)/4 + j.
 template<class F, bool kAligned>
@@ -36,9 +63,11 @@ __global__ void __launch_bounds__(kBlock) philox_fill(PhiloxCall a, F f)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const F g = stage_table(f, smem);
+    if(philox_edges(a, g))
+        return;
 
     const unsigned long long tid    = static_cast<unsigned long long>(blockIdx.x) * kBlock + threadIdx.x;
-    const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * kBlock;
+    const unsigned long long stride = static_cast<unsigned long long>(philox_blocks(a)) * kBlock;
 
     if(kAligned)
     {
@@ -64,32 +93,27 @@ __global__ void __launch_bounds__(kBlock) philox_fill(PhiloxCall a, F f)
         }
     }
 
-    if(tid == 0)
-    {
-        using T = typename F::T;
-        if(a.head > 0)
-            philox_scalar_run(a, g, 0, reinterpret_cast<T*>(a.data), a.head);
-        if(a.tail > 0)
-        {
-            const unsigned long long pos
-                = 4 * a.vec_n + ((a.vec_n % kPhiloxRefStride) == 0 ? a.start0 : a.head);
-            philox_scalar_run(a, g, pos, reinterpret_cast<T*>(a.data) + (a.n - a.tail), a.tail);
-        }
-    }
 }
 
 // Fast path: aligned vectors whose counters (x0 + j, y, z, w) share the upper words for the
 // whole launch (x0 + vec_n <= 2^32, checked by the host).  Each thread produces two
 // independent vectors per iteration so the two multiply chains interleave.
-template<class F>
+// kEdges: the call has a head or tail (a kernel of its own, because code for them in this one
+// changes the schedule of its loop: 2^26 uniform fp64 91.6 -> 95.7 us on one B200).
+template<bool kEdges, class F>
 __global__ void __launch_bounds__(kBlock)
     philox_fill_fast(PhiloxCall a, PhiloxLane lane, uint32_t x0, F f)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const F g = stage_table(f, smem);
+    if constexpr(kEdges)
+    {
+        if(philox_edges(a, g))
+            return;
+    }
 
     const uint32_t vec_n  = static_cast<uint32_t>(a.vec_n);
-    const uint32_t stride = gridDim.x * kBlock;
+    const uint32_t stride = (kEdges ? gridDim.x - 1 : gridDim.x) * kBlock;
     uint32_t       j      = blockIdx.x * kBlock + threadIdx.x;
     for(; j + stride < vec_n; j += 2 * stride)
     {
@@ -104,15 +128,72 @@ __global__ void __launch_bounds__(kBlock)
     if(j < vec_n)
         store16_cs(a.vec + static_cast<size_t>(j) * 16, philox_vec(g, philox_block_lane(x0 + j, lane, a.keys)));
 
-    if(blockIdx.x == 0 && threadIdx.x == 0)
+}
+
+// Shifted path: vectors whose words begin s = 1, 2 or 3 into a block (a misaligned buffer, or an
+// earlier call that ended inside a block), the upper counter words fixed as in the fast path
+// (x0 + vec_n + 1 <= 2^32, checked by the host).  A vector needs the last words of its block and
+// the first s of the next: a warp evaluates the blocks of kRows rows of 32 vectors and one more,
+// and every lane takes its neighbour's words by shuffle, so a vector costs 1 + 1/kRows
+// evaluations and s shuffles instead of two evaluations.  Vectors j % 262144 == 0 that begin
+// elsewhere (start0 != head) go through the general rule.  2^26 values one element off on one
+// B200, both blocks evaluated -> this: uint 115.9 -> 61.5 us, uniform fp64 230.7 -> 126.8, normal
+// fp32 170.4 -> 116.3.
+template<unsigned kRows, class F>
+__global__ void __launch_bounds__(kBlock)
+    philox_fill_shifted(PhiloxCall a, PhiloxLane lane, uint32_t x0, F f)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    const F g = stage_table(f, smem);
+    if(philox_edges(a, g))
+        return;
+
+    const uint32_t vec_n = static_cast<uint32_t>(a.vec_n);
+    const uint32_t s     = (a.s0 + a.head) & 3u;
+    const uint32_t l     = threadIdx.x & 31u;
+    const uint32_t step  = philox_blocks(a) * (kBlock / 32) * (32 * kRows);
+    const bool     odd   = a.start0 != a.head;
+    // `base` is the same in the whole warp: every lane takes part in the shuffles
+    for(uint32_t base = (blockIdx.x * (kBlock / 32) + threadIdx.x / 32) * (32 * kRows); base < vec_n; base += step)
     {
-        using T = typename F::T;
-        if(a.head > 0)
-            philox_scalar_run(a, g, 0, reinterpret_cast<T*>(a.data), a.head);
-        if(a.tail > 0)
-            philox_scalar_run(a, g, 4 * a.vec_n + a.head, reinterpret_cast<T*>(a.data) + (a.n - a.tail),
-                              a.tail);
+        uint4 b[kRows + 1];
+#pragma unroll
+        for(unsigned k = 0; k < kRows; k++)
+            b[k] = philox_block_lane(x0 + base + 32 * k + l, lane, a.keys);
+        b[kRows] = philox_block_lane(x0 + base + 32 * kRows, lane, a.keys); // lane 0's of the next row
+#pragma unroll
+        for(unsigned k = 0; k < kRows; k++)
+        {
+            // lane 31's neighbour is lane 0 one row on
+            const uint4    from = l == 0 ? b[k + 1] : b[k];
+            const unsigned src  = (l + 1) & 31u;
+            uint4          next = make_uint4(0u, 0u, 0u, 0u);
+            next.x              = __shfl_sync(0xffffffffu, from.x, src);
+            if(s > 1)
+                next.y = __shfl_sync(0xffffffffu, from.y, src);
+            if(s > 2)
+                next.z = __shfl_sync(0xffffffffu, from.z, src);
+            b[k] = interleave4(b[k], next, s);
+        }
+#pragma unroll
+        for(unsigned k = 0; k < kRows; k++)
+        {
+            const uint32_t j = base + 32 * k + l;
+            if(j >= vec_n)
+                break;
+            uint4 w = b[k];
+            if(odd && (j & (kPhiloxRefStride - 1)) == 0)
+            {
+                const unsigned long long q = a.s0 + a.start0 + 4ull * j;
+                const uint4              c = ctr_add(a.c0, q >> 2);
+                w                          = philox_block(c, a.keys);
+                if((q & 3) != 0)
+                    w = interleave4(w, philox_block(ctr_add(c, 1), a.keys), static_cast<uint32_t>(q & 3));
+            }
+            store16_cs(a.vec + static_cast<size_t>(j) * 16, philox_vec(g, w));
+        }
     }
+
 }
 
 // The same output contract on the host (host generators without a GPU): every vector by
@@ -145,32 +226,59 @@ static rocrand_status philox_run_host(const PhiloxCall& a, const F& f)
     return ROCRAND_STATUS_SUCCESS;
 }
 
+// Grid of a kernel over `work` threads' items, and the edges' block where there are any; all
+// resident at once.
+template<class Kernel>
+static unsigned philox_grid(Kernel k, const PhiloxCall& a, unsigned long long work, size_t smem)
+{
+    const unsigned edges = a.head + a.tail == 0 ? 0u : 1u;
+    const unsigned main  = grid_for(k, work > 0 ? work : 1, smem, edges);
+    return main + edges;
+}
+
 template<class F>
 static rocrand_status launch_philox(PhiloxCall a, const F& f, cudaStream_t stream)
 {
-    const size_t smem    = table_smem_bytes(f);
-    const bool   aligned = a.start0 == a.head && ((a.s0 + a.head) & 3u) == 0;
-    const unsigned long long work = a.vec_n > 0 ? a.vec_n : 1;
-    if(aligned)
+    const size_t   smem  = table_smem_bytes(f);
+    const uint32_t s     = (a.s0 + a.head) & 3u;
+    const uint4    cbase = ctr_add(a.c0, (a.s0 + a.head) >> 2);
+    // 32-bit indices in the fast kernels: keep j + 2*stride below 2^32 too.
+    const bool small = a.vec_n < (1ull << 31);
+    if(s == 0 && a.start0 == a.head)
     {
-        const uint4 cbase = ctr_add(a.c0, (a.s0 + a.head) >> 2);
-        // 32-bit indices in the fast kernel: keep j + 2*stride below 2^32 too.
-        if(static_cast<unsigned long long>(cbase.x) + a.vec_n <= (1ull << 32)
-           && a.vec_n < (1ull << 31))
+        if(static_cast<unsigned long long>(cbase.x) + a.vec_n <= (1ull << 32) && small)
         {
             const PhiloxLane lane = philox_lane(cbase, a.keys);
-            auto             k    = philox_fill_fast<F>;
-            k<<<grid_for(k, (work + 1) / 2, smem), kBlock, smem, stream>>>(a, lane, cbase.x, f);
+            auto             k    = a.head + a.tail == 0 ? philox_fill_fast<false, F> : philox_fill_fast<true, F>;
+            k<<<philox_grid(k, a, (a.vec_n + 1) / 2, smem), kBlock, smem, stream>>>(a, lane, cbase.x, f);
             return launch_status();
         }
         auto k = philox_fill<F, true>;
-        k<<<grid_for(k, work, smem), kBlock, smem, stream>>>(a, f);
+        k<<<philox_grid(k, a, a.vec_n, smem), kBlock, smem, stream>>>(a, f);
+        return launch_status();
     }
-    else
+    // Rows per warp of the shifted kernel, on one B200: from 2^20 vectors four fill the GPU (2^24
+    // values of normal fp32: 45.7 us evaluating every block twice, 35.7 with two rows, 31.4 with
+    // four); below that two (10^6 values of uniform fp32: 5.1, 4.1, 4.5); below 2^17 a thread's
+    // longer chain costs more than the evaluations saved (2^14 normal fp32: 4.1, 4.4, 6.2).
+    if(s != 0 && static_cast<unsigned long long>(cbase.x) + a.vec_n + 1 <= (1ull << 32) && small
+       && a.vec_n >= (1ull << 17))
     {
-        auto k = philox_fill<F, false>;
-        k<<<grid_for(k, work, smem), kBlock, smem, stream>>>(a, f);
+        const PhiloxLane lane = philox_lane(cbase, a.keys);
+        if(a.vec_n >= (1ull << 20))
+        {
+            auto k = philox_fill_shifted<4, F>;
+            k<<<philox_grid(k, a, (a.vec_n + 3) / 4, smem), kBlock, smem, stream>>>(a, lane, cbase.x, f);
+        }
+        else
+        {
+            auto k = philox_fill_shifted<2, F>;
+            k<<<philox_grid(k, a, (a.vec_n + 1) / 2, smem), kBlock, smem, stream>>>(a, lane, cbase.x, f);
+        }
+        return launch_status();
     }
+    auto k = philox_fill<F, false>;
+    k<<<philox_grid(k, a, a.vec_n, smem), kBlock, smem, stream>>>(a, f);
     return launch_status();
 }
 

@@ -58,15 +58,18 @@ __host__ __device__ __forceinline__ uint4 philox_vec(const F& f, uint4 w)
     constexpr unsigned opt = 4 / F::iw;
     typename F::T      out[opt * F::ow];
     const uint32_t     in[4] = {w.x, w.y, w.z, w.w};
-    if constexpr(opt == 1)
+    if constexpr(has_pair<F>::value)
     {
-        f(in, out);
+        static_assert(opt % 2 == 0, "pairs of units");
+#pragma unroll
+        for(unsigned s = 0; s < opt; s += 2)
+            f.pair(in + s * F::iw, in + (s + 1) * F::iw, out + s * F::ow, out + (s + 1) * F::ow);
     }
     else
     {
 #pragma unroll
-        for(unsigned s = 0; s < opt; s += 2)
-            apply_pair(f, in + s * F::iw, in + (s + 1) * F::iw, out + s * F::ow, out + (s + 1) * F::ow);
+        for(unsigned s = 0; s < opt; s++)
+            f(in + s * F::iw, out + s * F::ow);
     }
     return pack16(out);
 }
