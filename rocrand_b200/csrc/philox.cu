@@ -98,22 +98,17 @@ __global__ void __launch_bounds__(kBlock) philox_fill(PhiloxCall a, F f)
 // Fast path: aligned vectors whose counters (x0 + j, y, z, w) share the upper words for the
 // whole launch (x0 + vec_n <= 2^32, checked by the host).  Each thread produces two
 // independent vectors per iteration so the two multiply chains interleave.
-// kEdges: the call has a head or tail (a kernel of its own, because code for them in this one
-// changes the schedule of its loop: 2^26 uniform fp64 91.6 -> 95.7 us on one B200).
-template<bool kEdges, class F>
+// (Its head and tail stay behind block 0's vectors: a block of their own, as the other kernels
+// have, changes the schedule of this loop, 2^26 uniform fp64 91.6 -> 95.7 us on one B200.)
+template<class F>
 __global__ void __launch_bounds__(kBlock)
     philox_fill_fast(PhiloxCall a, PhiloxLane lane, uint32_t x0, F f)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const F g = stage_table(f, smem);
-    if constexpr(kEdges)
-    {
-        if(philox_edges(a, g))
-            return;
-    }
 
     const uint32_t vec_n  = static_cast<uint32_t>(a.vec_n);
-    const uint32_t stride = (kEdges ? gridDim.x - 1 : gridDim.x) * kBlock;
+    const uint32_t stride = gridDim.x * kBlock;
     uint32_t       j      = blockIdx.x * kBlock + threadIdx.x;
     for(; j + stride < vec_n; j += 2 * stride)
     {
@@ -128,6 +123,15 @@ __global__ void __launch_bounds__(kBlock)
     if(j < vec_n)
         store16_cs(a.vec + static_cast<size_t>(j) * 16, philox_vec(g, philox_block_lane(x0 + j, lane, a.keys)));
 
+    if(blockIdx.x == 0 && threadIdx.x == 0)
+    {
+        using T = typename F::T;
+        if(a.head > 0)
+            philox_scalar_run(a, g, 0, reinterpret_cast<T*>(a.data), a.head);
+        if(a.tail > 0)
+            philox_scalar_run(a, g, 4 * a.vec_n + a.head, reinterpret_cast<T*>(a.data) + (a.n - a.tail),
+                              a.tail);
+    }
 }
 
 // Shifted path: vectors whose words begin s = 1, 2 or 3 into a block (a misaligned buffer, or an
@@ -249,8 +253,8 @@ static rocrand_status launch_philox(PhiloxCall a, const F& f, cudaStream_t strea
         if(static_cast<unsigned long long>(cbase.x) + a.vec_n <= (1ull << 32) && small)
         {
             const PhiloxLane lane = philox_lane(cbase, a.keys);
-            auto             k    = a.head + a.tail == 0 ? philox_fill_fast<false, F> : philox_fill_fast<true, F>;
-            k<<<philox_grid(k, a, (a.vec_n + 1) / 2, smem), kBlock, smem, stream>>>(a, lane, cbase.x, f);
+            auto             k    = philox_fill_fast<F>;
+            k<<<grid_for(k, a.vec_n > 0 ? (a.vec_n + 1) / 2 : 1, smem), kBlock, smem, stream>>>(a, lane, cbase.x, f);
             return launch_status();
         }
         auto k = philox_fill<F, true>;
