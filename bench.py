@@ -73,9 +73,9 @@ NCU_INST = {
     ("philox4x32_10", "uniform"): 0.4155,
     ("philox4x32_10", "uniform_double"): 0.8292,
     ("philox4x32_10", "uniform_half"): 0.2744,
-    ("philox4x32_10", "normal[0.0, 1.0]"): 1.6415,
-    ("philox4x32_10", "normal_double[0.0, 1.0]"): 4.2097,
-    ("philox4x32_10", "log_normal[0.0, 1.0]"): 1.9227,
+    ("philox4x32_10", "normal[0.0, 1.0]"): 0.9659,
+    ("philox4x32_10", "normal_double[0.0, 1.0]"): 2.8615,
+    ("philox4x32_10", "log_normal[0.0, 1.0]"): 1.2004,
     ("philox4x32_10", "poisson[0.5]"): 0.6473,
     ("philox4x32_10", "poisson[10.0]"): 0.6482,
     ("philox4x32_10", "poisson[1000.0]"): 0.6567,
@@ -83,102 +83,102 @@ NCU_INST = {
     ("xorwow", "uniform"): 0.3970,
     ("xorwow", "uniform_double"): 0.6548,
     ("xorwow", "uniform_half"): 0.2766,
-    ("xorwow", "normal[0.0, 1.0]"): 1.5476,
-    ("xorwow", "normal_double[0.0, 1.0]"): 3.9299,
-    ("xorwow", "log_normal[0.0, 1.0]"): 1.8289,
-    ("xorwow", "poisson[0.5]"): 0.6151,
-    ("xorwow", "poisson[10.0]"): 0.6155,
-    ("xorwow", "poisson[1000.0]"): 0.6190,
-    ("mrg32k3a", "uint"): 1.2554,
-    ("mrg32k3a", "uniform"): 1.2395,
-    ("mrg32k3a", "uniform_double"): 1.2139,
-    ("mrg32k3a", "uniform_half"): 0.7507,
-    ("mrg32k3a", "normal[0.0, 1.0]"): 2.4856,
-    ("mrg32k3a", "normal_double[0.0, 1.0]"): 4.6174,
-    ("mrg32k3a", "log_normal[0.0, 1.0]"): 2.7668,
-    ("mrg32k3a", "poisson[0.5]"): 1.5675,
-    ("mrg32k3a", "poisson[10.0]"): 1.5679,
-    ("mrg32k3a", "poisson[1000.0]"): 1.5714,
+    ("xorwow", "normal[0.0, 1.0]"): 0.8877,
+    ("xorwow", "normal_double[0.0, 1.0]"): 2.5496,
+    ("xorwow", "log_normal[0.0, 1.0]"): 1.1155,
+    ("xorwow", "poisson[0.5]"): 0.6155,
+    ("xorwow", "poisson[10.0]"): 0.6163,
+    ("xorwow", "poisson[1000.0]"): 0.6220,
+    ("mrg32k3a", "uint"): 1.1257,
+    ("mrg32k3a", "uniform"): 1.0730,
+    ("mrg32k3a", "uniform_double"): 1.0325,
+    ("mrg32k3a", "uniform_half"): 0.7056,
+    ("mrg32k3a", "normal[0.0, 1.0]"): 1.5955,
+    ("mrg32k3a", "normal_double[0.0, 1.0]"): 3.1768,
+    ("mrg32k3a", "log_normal[0.0, 1.0]"): 1.8611,
+    ("mrg32k3a", "poisson[0.5]"): 1.4100,
+    ("mrg32k3a", "poisson[10.0]"): 1.4107,
+    ("mrg32k3a", "poisson[1000.0]"): 1.4164,
     ("lfsr113", "uint"): 0.7690,
     ("lfsr113", "uniform"): 0.8394,
     ("lfsr113", "uniform_double"): 1.5347,
     ("lfsr113", "uniform_half"): 0.4895,
-    ("lfsr113", "normal[0.0, 1.0]"): 1.9692,
-    ("lfsr113", "normal_double[0.0, 1.0]"): 4.7683,
-    ("lfsr113", "log_normal[0.0, 1.0]"): 2.2505,
-    ("lfsr113", "poisson[0.5]"): 1.0531,
-    ("lfsr113", "poisson[10.0]"): 1.0535,
-    ("lfsr113", "poisson[1000.0]"): 1.0570,
-    ("mt19937", "uint"): 0.8396,
-    ("mt19937", "uniform"): 0.9146,
-    ("mt19937", "uniform_double"): 1.3757,
-    ("mt19937", "uniform_half"): 0.6749,
-    ("mt19937", "normal[0.0, 1.0]"): 2.2219,
-    ("mt19937", "normal_double[0.0, 1.0]"): 4.9500,
-    ("mt19937", "log_normal[0.0, 1.0]"): 2.5032,
-    ("mt19937", "poisson[0.5]"): 1.1601,
-    ("mt19937", "poisson[10.0]"): 1.1608,
-    ("mt19937", "poisson[1000.0]"): 1.1660,
-    ("threefry4x32_20", "uint"): 1.1911,
-    ("threefry4x32_20", "uniform"): 1.2614,
-    ("threefry4x32_20", "uniform_double"): 2.5036,
-    ("threefry4x32_20", "uniform_half"): 0.6872,
-    ("threefry4x32_20", "normal[0.0, 1.0]"): 2.4985,
-    ("threefry4x32_20", "normal_double[0.0, 1.0]"): 5.7965,
-    ("threefry4x32_20", "log_normal[0.0, 1.0]"): 2.7797,
-    ("threefry4x32_20", "poisson[0.5]"): 1.4929,
-    ("threefry4x32_20", "poisson[10.0]"): 1.4938,
-    ("threefry4x32_20", "poisson[1000.0]"): 1.5023,
-    ("mtgp32", "uint"): 1.1253,
-    ("mtgp32", "uniform"): 1.1956,
-    ("mtgp32", "uniform_double"): 2.9434,
-    ("mtgp32", "uniform_half"): 0.8387,
-    ("mtgp32", "normal[0.0, 1.0]"): 2.4131,
-    ("mtgp32", "normal_double[0.0, 1.0]"): 5.4471,
-    ("mtgp32", "log_normal[0.0, 1.0]"): 2.6944,
-    ("mtgp32", "poisson[0.5]"): 1.7156,
-    ("mtgp32", "poisson[10.0]"): 1.7160,
-    ("mtgp32", "poisson[1000.0]"): 1.7199,
-    ("mrg31k3p", "uint"): 1.4998,
+    ("lfsr113", "normal[0.0, 1.0]"): 1.3159,
+    ("lfsr113", "normal_double[0.0, 1.0]"): 3.4363,
+    ("lfsr113", "log_normal[0.0, 1.0]"): 1.5425,
+    ("lfsr113", "poisson[0.5]"): 1.0535,
+    ("lfsr113", "poisson[10.0]"): 1.0543,
+    ("lfsr113", "poisson[1000.0]"): 1.0600,
+    ("mt19937", "uint"): 0.8389,
+    ("mt19937", "uniform"): 0.9138,
+    ("mt19937", "uniform_double"): 1.3754,
+    ("mt19937", "uniform_half"): 0.6746,
+    ("mt19937", "normal[0.0, 1.0]"): 1.3821,
+    ("mt19937", "normal_double[0.0, 1.0]"): 3.4446,
+    ("mt19937", "log_normal[0.0, 1.0]"): 1.6105,
+    ("mt19937", "poisson[0.5]"): 1.1594,
+    ("mt19937", "poisson[10.0]"): 1.1601,
+    ("mt19937", "poisson[1000.0]"): 1.1652,
+    ("threefry4x32_20", "uint"): 1.0856,
+    ("threefry4x32_20", "uniform"): 1.1559,
+    ("threefry4x32_20", "uniform_double"): 2.2809,
+    ("threefry4x32_20", "uniform_half"): 0.6324,
+    ("threefry4x32_20", "normal[0.0, 1.0]"): 1.7195,
+    ("threefry4x32_20", "normal_double[0.0, 1.0]"): 4.4337,
+    ("threefry4x32_20", "log_normal[0.0, 1.0]"): 1.9617,
+    ("threefry4x32_20", "poisson[0.5]"): 1.3801,
+    ("threefry4x32_20", "poisson[10.0]"): 1.3809,
+    ("threefry4x32_20", "poisson[1000.0]"): 1.3889,
+    ("mtgp32", "uint"): 0.9520,
+    ("mtgp32", "uniform"): 1.0223,
+    ("mtgp32", "uniform_double"): 1.9598,
+    ("mtgp32", "uniform_half"): 0.5785,
+    ("mtgp32", "normal[0.0, 1.0]"): 1.5702,
+    ("mtgp32", "normal_double[0.0, 1.0]"): 3.7053,
+    ("mtgp32", "log_normal[0.0, 1.0]"): 1.8119,
+    ("mtgp32", "poisson[0.5]"): 1.2440,
+    ("mtgp32", "poisson[10.0]"): 1.2444,
+    ("mtgp32", "poisson[1000.0]"): 1.2483,
+    ("mrg31k3p", "uint"): 1.5300,
     ("mrg31k3p", "uniform"): 1.4685,
     ("mrg31k3p", "uniform_double"): 1.4363,
-    ("mrg31k3p", "uniform_half"): 0.8748,
-    ("mrg31k3p", "normal[0.0, 1.0]"): 2.6685,
-    ("mrg31k3p", "normal_double[0.0, 1.0]"): 4.8044,
-    ("mrg31k3p", "log_normal[0.0, 1.0]"): 2.9497,
-    ("mrg31k3p", "poisson[0.5]"): 1.7848,
-    ("mrg31k3p", "poisson[10.0]"): 1.7852,
-    ("mrg31k3p", "poisson[1000.0]"): 1.7887,
-    ("threefry2x32_20", "uint"): 1.2033,
-    ("threefry2x32_20", "uniform"): 1.2814,
-    ("threefry2x32_20", "uniform_double"): 2.5471,
-    ("threefry2x32_20", "uniform_half"): 0.6955,
-    ("threefry2x32_20", "normal[0.0, 1.0]"): 2.6073,
-    ("threefry2x32_20", "normal_double[0.0, 1.0]"): 5.9723,
-    ("threefry2x32_20", "log_normal[0.0, 1.0]"): 2.8886,
-    ("threefry2x32_20", "poisson[0.5]"): 1.4889,
-    ("threefry2x32_20", "poisson[10.0]"): 1.4899,
-    ("threefry2x32_20", "poisson[1000.0]"): 1.4983,
-    ("threefry2x64_20", "uint"): 1.2759,
-    ("threefry2x64_20", "uniform"): 2.6118,
-    ("threefry2x64_20", "uniform_double"): 2.6899,
-    ("threefry2x64_20", "uniform_half"): 0.7368,
-    ("threefry2x64_20", "normal[0.0, 1.0]"): 2.6313,
-    ("threefry2x64_20", "normal_double[0.0, 1.0]"): 6.1530,
-    ("threefry2x64_20", "log_normal[0.0, 1.0]"): 2.9126,
-    ("threefry2x64_20", "poisson[0.5]"): 2.9953,
-    ("threefry2x64_20", "poisson[10.0]"): 2.9963,
-    ("threefry2x64_20", "poisson[1000.0]"): 3.0074,
-    ("threefry4x64_20", "uint"): 1.2798,
-    ("threefry4x64_20", "uniform"): 2.6001,
-    ("threefry4x64_20", "uniform_double"): 2.6783,
-    ("threefry4x64_20", "uniform_half"): 0.7388,
-    ("threefry4x64_20", "normal[0.0, 1.0]"): 2.6241,
-    ("threefry4x64_20", "normal_double[0.0, 1.0]"): 6.1164,
-    ("threefry4x64_20", "log_normal[0.0, 1.0]"): 2.9053,
-    ("threefry4x64_20", "poisson[0.5]"): 3.0316,
-    ("threefry4x64_20", "poisson[10.0]"): 3.0327,
-    ("threefry4x64_20", "poisson[1000.0]"): 3.0437,
+    ("mrg31k3p", "uniform_half"): 0.9065,
+    ("mrg31k3p", "normal[0.0, 1.0]"): 1.9756,
+    ("mrg31k3p", "normal_double[0.0, 1.0]"): 3.5137,
+    ("mrg31k3p", "log_normal[0.0, 1.0]"): 2.2412,
+    ("mrg31k3p", "poisson[0.5]"): 1.8170,
+    ("mrg31k3p", "poisson[10.0]"): 1.8177,
+    ("mrg31k3p", "poisson[1000.0]"): 1.8234,
+    ("threefry2x32_20", "uint"): 1.1681,
+    ("threefry2x32_20", "uniform"): 1.2462,
+    ("threefry2x32_20", "uniform_double"): 2.4800,
+    ("threefry2x32_20", "uniform_half"): 0.6754,
+    ("threefry2x32_20", "normal[0.0, 1.0]"): 1.7956,
+    ("threefry2x32_20", "normal_double[0.0, 1.0]"): 5.7340,
+    ("threefry2x32_20", "log_normal[0.0, 1.0]"): 2.0385,
+    ("threefry2x32_20", "poisson[0.5]"): 1.4554,
+    ("threefry2x32_20", "poisson[10.0]"): 1.4562,
+    ("threefry2x32_20", "poisson[1000.0]"): 1.4642,
+    ("threefry2x64_20", "uint"): 1.1687,
+    ("threefry2x64_20", "uniform"): 2.4030,
+    ("threefry2x64_20", "uniform_double"): 2.4812,
+    ("threefry2x64_20", "uniform_half"): 0.6804,
+    ("threefry2x64_20", "normal[0.0, 1.0]"): 1.8356,
+    ("threefry2x64_20", "normal_double[0.0, 1.0]"): 4.7283,
+    ("threefry2x64_20", "log_normal[0.0, 1.0]"): 2.1012,
+    ("threefry2x64_20", "poisson[0.5]"): 2.8038,
+    ("threefry2x64_20", "poisson[10.0]"): 2.8049,
+    ("threefry2x64_20", "poisson[1000.0]"): 2.8159,
+    ("threefry4x64_20", "uint"): 1.1085,
+    ("threefry4x64_20", "uniform"): 2.2570,
+    ("threefry4x64_20", "uniform_double"): 2.3351,
+    ("threefry4x64_20", "uniform_half"): 0.6534,
+    ("threefry4x64_20", "normal[0.0, 1.0]"): 1.7508,
+    ("threefry4x64_20", "normal_double[0.0, 1.0]"): 4.4156,
+    ("threefry4x64_20", "log_normal[0.0, 1.0]"): 2.0165,
+    ("threefry4x64_20", "poisson[0.5]"): 2.6511,
+    ("threefry4x64_20", "poisson[10.0]"): 2.6521,
+    ("threefry4x64_20", "poisson[1000.0]"): 2.6631,
 }
 
 
