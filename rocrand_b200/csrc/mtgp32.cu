@@ -78,8 +78,8 @@ static_assert(kMtgpBlock + kMtgpReach <= kMtgpN, "a step reads no word that it w
 // values: 66.7 us for 2^26 values on an SM with four of the 512 generators; the rest is the
 // chain of a step (load, table, store, barrier), which four blocks overlap only in part.  With
 // the offsets wrapped by masks at run time, each step was 36 instructions a value.  2^26 values
-// on one B200, before -> now: uniform fp32 112.7 -> 100.4 us, uniform fp64 274 -> 198, normal
-// fp32 (packed transform either way) 165 -> 153, fp64 468 either way, Poisson 168 -> 133.
+// on one B200, before -> now (the transforms' own changes included): uniform fp32 113 -> 97..101
+// us, uniform fp64 273 -> 197, normal fp32 202 -> 151, fp64 541 -> 467, Poisson 167 -> 130.
 template<class F>
 __global__ void __launch_bounds__(kMtgpBlock, 4) mtgp_fill(MtgpArgs a, F fw)
 {
@@ -91,9 +91,18 @@ __global__ void __launch_bounds__(kMtgpBlock, 4) mtgp_fill(MtgpArgs a, F fw)
     const F                    f = stage_table(fw, smem);
     const uint32_t             b = blockIdx.x, t = threadIdx.x;
     const uint32_t*            p = a.params + b * kMtgpWords;
-    const int                  k = a.offsets[b];
-    for(int i = static_cast<int>(t); i < kMtgpState; i += kMtgpBlock)
-        s[i] = a.rings[b * kMtgpState + ((k + i) & kMtgpMask)];
+    // The ring's words and its offset are read side by side: reading the words at the offset
+    // made every call wait for memory twice (2^18 values on one B200: uniform half 6.15 -> 4.11
+    // us, uint 5.13 -> 4.12, Poisson 6.16 -> 4.13).
+    constexpr int              kLoads = kMtgpState / static_cast<int>(kMtgpBlock);
+    uint32_t                   ring[kLoads];
+#pragma unroll
+    for(int i = 0; i < kLoads; i++)
+        ring[i] = a.rings[b * kMtgpState + i * kMtgpBlock + t];
+    const int k = a.offsets[b];
+#pragma unroll
+    for(int i = 0; i < kLoads; i++)
+        s[(i * static_cast<int>(kMtgpBlock) + static_cast<int>(t) - k) & kMtgpMask] = ring[i];
     if(t < 16)
     {
         tbl[t] = p[3 + t];
