@@ -178,13 +178,30 @@ struct FillArgs
 // HBM) 51.3 -> 49.6; MRG32k3a uint 132.7 -> 118.3; LFSR113 uint 73.5 -> 64.6.
 constexpr unsigned kFillBlock = 128;
 
+// The same where a warp's stores begin and end inside a 32-byte sector (a misaligned buffer) and
+// the output is larger than L2: a sector that two blocks share is written twice to memory when
+// they have drifted apart, so wide blocks, with a fourth of the shared sectors, are the faster
+// ones for the kinds whose stores bound them.  One value off, 2^28 values a call on one B200,
+// 128 -> 512 threads: XORWOW uint 425 -> 244 us, uint16 206 -> 131, uniform fp64 635 -> 502,
+// Poisson 432 -> 352 (2^26: 85 -> 58, 43 -> 34, 135 -> 110, 79 -> 63); MRG32k3a uniform fp64 660
+// -> 563, MRG31k3p's 655 -> 582; LFSR113 half 213 -> 157, uint16 207 -> 172.  The others do not
+// drift or are bound by issue, and lose (MRG32k3a uint 385 -> 440, LFSR113 uint 243 -> 307), as
+// all do within L2 (2^24 XORWOW uint 16.6 -> 17.1).
+constexpr unsigned kWideFillBlock = 512;
+constexpr size_t   kWideFillBytes = size_t(128) << 20;
 template<class E, class F>
-__global__ void __launch_bounds__(kFillBlock) stateful_fill(FillArgs a, F f)
+constexpr bool kWideFill
+    = !long_transform<F>::value && !std::is_same_v<F, FnPoissonHuge>
+      && (std::is_same_v<E, XorwowEngine> || (std::is_same_v<E, Lfsr113Engine> && sizeof(typename F::T) <= 2)
+          || (!std::is_same_v<E, Lfsr113Engine> && sizeof(typename F::T) == 8 && F::ow == 1)); // uniform fp64
+
+template<unsigned kThreads, class E, class F>
+__global__ void __launch_bounds__(kThreads) stateful_fill(FillArgs a, F f)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const F g = stage_table(f, smem);
 
-    const uint32_t t = blockIdx.x * kFillBlock + threadIdx.x; // slot
+    const uint32_t t = blockIdx.x * kThreads + threadIdx.x; // slot
     if(t >= kE)
         return;
     const bool loops = t < a.vec_n;
@@ -967,8 +984,16 @@ private:
             const size_t smem = table_smem_bytes(f);
             // the slots that write: vector j's is j mod E, and the edges' follows the last vector
             const unsigned long long slots = std::min<unsigned long long>(a.vec_n + 1, kE);
-            const unsigned           grid  = static_cast<unsigned>((slots + kFillBlock - 1) / kFillBlock);
-            stateful_fill<Eng, F><<<grid, kFillBlock, smem, m_stream>>>(a, f);
+            const auto               grid  = [&](unsigned b) { return static_cast<unsigned>((slots + b - 1) / b); };
+            bool                     wide  = false;
+            if constexpr(kWideFill<Eng, F>)
+            {
+                wide = reinterpret_cast<uintptr_t>(a.vec) % 32 != 0 && n >= kWideFillBytes / tsize;
+                if(wide)
+                    stateful_fill<kWideFillBlock, Eng><<<grid(kWideFillBlock), kWideFillBlock, smem, m_stream>>>(a, f);
+            }
+            if(!wide)
+                stateful_fill<kFillBlock, Eng><<<grid(kFillBlock), kFillBlock, smem, m_stream>>>(a, f);
             const rocrand_status st = launch_status();
             if(st != ROCRAND_STATUS_SUCCESS)
                 return st;
