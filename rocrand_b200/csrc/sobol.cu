@@ -79,31 +79,50 @@ inline unsigned long long sobol_chunk(unsigned long long n, unsigned long long d
 // leaves blocks out of the first wave.  Many short blocks in the order of memory keep the writes
 // of the moment together: plain stores of 1 GiB run at 7.2-7.4 TB/s in blocks of 28 to 112 KiB
 // and at 6.0-6.3 TB/s in one wave of long runs or grid strides, whose blocks drift apart.  64
-// dimensions, 2^26 uniform fp64 on one B200, by whole waves -> by 32 KiB: Sobol32 150 -> 137 us,
+// dimensions, 2^26 uniform fp64 on one B200, by whole waves -> by 32 KiB: Sobol32 150 -> 126 us,
 // scrambled Sobol64 157 -> 116 (2^24: 62.8 -> 34.6).  The 4-byte kinds gain nothing or lose
 // (uniform fp32 44.6 -> 49.3: a block's start costs them more) and keep whole waves.
-inline unsigned long long sobol_store_chunk(unsigned long long n, unsigned long long dims,
-                                            unsigned long long group, unsigned long long wave, size_t size)
+inline unsigned long long sobol_store_chunk(unsigned long long group, unsigned long long spread, size_t size)
 {
-    const unsigned long long full   = 32768 / (group * size);
-    const unsigned long long spread = (n + group - 1) / group * dims / (wave == 0 ? 1 : wave);
-    const unsigned long long per    = std::max<unsigned long long>(1, std::min(full, spread));
-    return per * group;
+    const unsigned long long full = 32768 / (group * size);
+    return std::max<unsigned long long>(1, std::min(full, spread)) * group;
 }
 
-// Blocks that an SM has to hold: all eight for the kinds that are little more than a store (with
-// seven, 64 dimensions x 2^20 uint32 were cut into 16 long runs a row, 1024 streams of one wave,
-// and took 86 us instead of 45 on one B200); the transforms may use the registers for the four
-// points they work on side by side.
 template<SobolKind K>
-constexpr unsigned kSobolBlocks = K == SobolKind::UINT || K == SobolKind::ULL || K == SobolKind::UCHAR
-                                          || K == SobolKind::USHORT || K == SobolKind::FLOAT
-                                          || K == SobolKind::DOUBLE || K == SobolKind::HALF
-                                      ? 8u
-                                      : 1u;
+constexpr bool kSobolStores = K == SobolKind::UINT || K == SobolKind::ULL || K == SobolKind::UCHAR
+                              || K == SobolKind::USHORT || K == SobolKind::FLOAT || K == SobolKind::DOUBLE
+                              || K == SobolKind::HALF;
 
+// Forms of the kernel: whether a thread looks every step's direction vector up or keeps three of
+// four in registers, and the blocks that an SM has to hold (0: as many as the registers leave).
+// Registers pay for the 64-bit sequences, whose lookups are 8 bytes; the 32-bit kinds lose
+// residency by them.  Measured on one B200, look up -> registers, the output buffer another one
+// each call:
+//  * Sobol32, 64 dimensions: 2^25 Poisson 97 -> 132 us, 2^24 half normals 70 -> 83; 1000
+//    dimensions of 272 normals 6.2 -> 8.2;
+//  * Sobol64, 64 dimensions x 2^20: normal fp32 289 -> 245 us, uint32 64 -> 56, uint8 77 -> 44.
+// The kinds that are little more than a store need all eight blocks (with seven, 64 dimensions x
+// 2^20 uint32 were cut into 16 long runs a row, 1024 streams of one wave, and took 86 us instead
+// of 45), except Sobol32's uniform fp64, which the cap costs more than a block (2^21 values 8.4
+// -> 6.6 us, 2^27 267 -> 246).  Poisson searches its table in shared memory, which residency
+// hides (Sobol64, 2^24 values: 87 us with the transforms' registers, 58 without).  The fp64
+// normals gain as much as they lose (Sobol32, 64 dimensions: 2^25 values 222 -> 205 us, 2^22 31.3
+// -> 33.2) and keep the registers.
 template<class W, SobolKind K>
-__global__ void __launch_bounds__(kBlock, kSobolBlocks<K>) sobol_fill(SobolCall<W> a)
+constexpr bool kSobolLook = sizeof(W) == 4 && K != SobolKind::NORMAL_D && K != SobolKind::LOGNORMAL_D;
+template<class W, SobolKind K>
+constexpr unsigned kSobolBlocks = kSobolStores<K> ? (sizeof(W) == 4 && K == SobolKind::DOUBLE ? 0u : 8u)
+                                                  : (kSobolLook<W, K> || K == SobolKind::POISSON ? 0u : 1u);
+
+// The 8-byte kinds have the other form too (the lookup of Sobol64 with free registers, Sobol32's
+// at eight blocks), for the calls that are not cut into short blocks of whole vectors.
+template<class W, SobolKind K>
+constexpr bool kSobolTwoForms = K == SobolKind::DOUBLE || (sizeof(W) == 8 && K == SobolKind::ULL);
+template<class W, SobolKind K>
+constexpr unsigned kSobolOtherBlocks = sizeof(W) == 4 ? 8u : 0u;
+
+template<class W, SobolKind K, bool kLook, unsigned kBlocks>
+__global__ void __launch_bounds__(kBlock, kBlocks) sobol_fill(SobolCall<W> a)
 {
     using T                = typename SobolOut<K, W>::T;
     constexpr int      B   = 8 * sizeof(W);
@@ -154,16 +173,14 @@ __global__ void __launch_bounds__(kBlock, kSobolBlocks<K>) sobol_fill(SobolCall<
     // Point i to i + 1 flips the direction vector of i's lowest zero bit: number 0, 1, 0 after
     // i = 0, 1, 2 (mod 4), and one to look up after i = 3 (mod 4).  A thread's points start at the
     // same residue every time (strides are multiples of 4), so of four steps three have their
-    // vector in a register.  (The 32-bit kinds that only store look every one up: their kernel
-    // waits for memory, and 2^26 uniform fp32 is 45 us that way and 48 this.)
-    constexpr bool kLookAll = sizeof(W) == 4 && kSobolBlocks<K> > 1;
+    // vector in a register unless kLook has every one looked up.
     const unsigned residue  = static_cast<unsigned>(i) & 3u;
     const W        v0 = v[0], v1 = v[1], vl = v[lg - 1];
     for(; p < end; p += stride)
     {
         T out[PPT];
         W look[PPT / 4];
-        if constexpr(!kLookAll)
+        if constexpr(!kLook)
         {
 #pragma unroll
             for(unsigned j = 0; j < PPT / 4; j++)
@@ -174,7 +191,7 @@ __global__ void __launch_bounds__(kBlock, kSobolBlocks<K>) sobol_fill(SobolCall<
         for(unsigned k = 0; k < PPT; k++)
         {
             out[k] = sobol_apply<K, W>(xx ^ c, a.p, cdf);
-            if constexpr(kLookAll)
+            if constexpr(kLook)
             {
                 xx ^= v[rzb(static_cast<I>(i + k))];
             }
@@ -370,6 +387,57 @@ public:
     }
 
 private:
+    // A launch shape (kind, points per dimension, shared memory, dimensions, rows of whole
+    // vectors) and what serves it, chosen once per shape.
+    using Kernel = void (*)(SobolCall<W>);
+    struct Plan
+    {
+        Kernel             kind   = nullptr;
+        unsigned long long n      = 0;
+        size_t             smem   = 0;
+        unsigned int       dims   = 0;
+        bool               whole  = false;
+        Kernel             kernel = nullptr;
+        unsigned long long chunk  = 0; // points per block
+    };
+
+    template<SobolKind K>
+    Plan plan(Kernel kind, unsigned long long n, size_t smem, bool whole) const
+    {
+        using T                            = typename SobolOut<K, W>::T;
+        constexpr unsigned           PPT   = sizeof(T) >= 4 ? 4u : 16u / sizeof(T);
+        constexpr unsigned long long group = static_cast<unsigned long long>(PPT) * kBlock;
+        const auto wave_of = [&](Kernel k) {
+            return static_cast<unsigned long long>(device_info().sm_count)
+                   * blocks_per_sm(reinterpret_cast<const void*>(k), smem);
+        };
+        Plan r{kind, n, smem, m_dims, whole, kind, 0};
+        if constexpr(kSobolTwoForms<W, K>)
+        {
+            // Short blocks, unless one group a block would be one wave and a part of the next
+            // (Sobol64, 2^21 uint64: 10.4 us that way, 7.2 by whole waves of the other form; 2^22:
+            // 10.6, 11.1), or the rows are not made of whole vectors and there are many (1000
+            // dimensions x 8389 points of Sobol64 uniform fp64: 37 us, 29; 3 dimensions of as many
+            // points in all: 33, 40).  Sobol32 keeps short blocks in the first case (6.6 us,
+            // 8.4); its other form is the faster one where vectors are split (64 dimensions x
+            // 32769 points of uniform fp64: 12.4 us, 10.5).
+            constexpr auto           other  = sobol_fill<W, K, true, kSobolOtherBlocks<W, K>>;
+            if(sizeof(W) == 4 && !whole)
+                r.kernel = other;
+            const unsigned long long spread = (n + group - 1) / group * m_dims / wave_of(r.kernel);
+            const bool               waves  = whole ? sizeof(W) == 8 && spread == 1 : m_dims >= 128 && spread >= 2;
+            if(sizeof(W) == 8 && waves)
+                r.kernel = other;
+            r.chunk = waves ? sobol_chunk(n, m_dims, group, wave_of(r.kernel))
+                            : sobol_store_chunk(group, spread, sizeof(T));
+        }
+        else
+        {
+            r.chunk = sobol_chunk(n, m_dims, group, wave_of(kind));
+        }
+        return r;
+    }
+
     template<SobolKind K>
     rocrand_status launch(void* data, size_t n, const SobolParams& p)
     {
@@ -391,25 +459,18 @@ private:
         a.offset   = m_current;
         a.p        = p;
         // blocks per dimension: whole groups of PPT * kBlock points each, as many as fill the
-        // GPU's resident blocks in nearly whole waves
-        const size_t             smem  = K == SobolKind::POISSON ? p.size * sizeof(double) : 0;
-        constexpr unsigned long long group = static_cast<unsigned long long>(PPT) * kBlock;
-        const void* const kernel = reinterpret_cast<const void*>(sobol_fill<W, K>);
-        if(m_chunk_kernel != kernel || m_chunk_n != N || m_chunk_smem != smem || m_chunk_dims != m_dims)
-        {
-            const unsigned long long wave
-                = static_cast<unsigned long long>(device_info().sm_count) * blocks_per_sm(kernel, smem);
-            m_chunk        = K == SobolKind::DOUBLE || K == SobolKind::ULL
-                                 ? sobol_store_chunk(N, m_dims, group, wave, sizeof(T))
-                                 : sobol_chunk(N, m_dims, group, wave);
-            m_chunk_kernel = kernel;
-            m_chunk_n      = N;
-            m_chunk_smem   = smem;
-            m_chunk_dims   = m_dims;
-        }
-        a.chunk                        = m_chunk;
-        const unsigned long long nb    = (N + a.chunk - 1) / a.chunk;
-        sobol_fill<W, K><<<dim3(static_cast<unsigned>(nb), m_dims), kBlock, smem, m_stream>>>(a);
+        // GPU's resident blocks in nearly whole waves, or short blocks (the 8-byte kinds that
+        // only store)
+        const size_t   smem   = K == SobolKind::POISSON ? p.size * sizeof(double) : 0;
+        constexpr auto kernel = sobol_fill<W, K, kSobolLook<W, K>, kSobolBlocks<W, K>>;
+        const bool     whole  = reinterpret_cast<uintptr_t>(data) % (PPT * sizeof(T)) == 0
+                           && (m_dims == 1 || N * sizeof(T) % (PPT * sizeof(T)) == 0);
+        if(m_plan.kind != kernel || m_plan.n != N || m_plan.smem != smem || m_plan.dims != m_dims
+           || m_plan.whole != whole)
+            m_plan = plan<K>(kernel, N, smem, whole);
+        a.chunk                     = m_plan.chunk;
+        const unsigned long long nb = (N + a.chunk - 1) / a.chunk;
+        m_plan.kernel<<<dim3(static_cast<unsigned>(nb), m_dims), kBlock, smem, m_stream>>>(a);
         return launch_status();
     }
 
@@ -462,13 +523,7 @@ private:
     unsigned int       m_dims        = 1;
     bool               m_initialized = false;
     PoissonCache       m_poisson;
-    // the block size in points of the last launch shape (kernel, points per dimension,
-    // shared memory, dimensions), chosen once per shape
-    const void*        m_chunk_kernel = nullptr;
-    unsigned long long m_chunk_n      = 0;
-    size_t             m_chunk_smem   = 0;
-    unsigned int       m_chunk_dims   = 0;
-    unsigned long long m_chunk        = 0;
+    Plan               m_plan;
 };
 
 rocrand_generator_base_type* make_sobol(rocrand_rng_type t)
