@@ -47,19 +47,43 @@ def torch_dtype(dist):
             np.float16: torch.float16}[dt]
 
 
+GUARD = 512        # guard bytes on each side of an output (a multiple of every alignment)
+GUARD_BYTE = 0xA5  # what they hold
+
+
+def guarded_output(n, dtype, mis=0, device="cuda"):
+    """A buffer full of GUARD_BYTE and the n elements in its middle, (mis * itemsize) bytes past a
+    512-byte boundary of the buffer: (buffer as bytes, output as a tensor of `dtype`, its address)."""
+    import torch
+    isz = torch.empty(0, dtype=dtype).element_size()
+    at = GUARD + mis * isz
+    raw = torch.full(((at + n * isz + GUARD + 15) // 16 * 16,), GUARD_BYTE, dtype=torch.uint8, device=device)
+    return raw, raw[at:at + n * isz].view(dtype), raw.data_ptr() + at
+
+
+def check_guards(raw, out):
+    """Asserts that nothing around `out` in `raw` was written."""
+    at = out.storage_offset() * out.element_size()
+    end = at + out.numel() * out.element_size()
+    for name, part in (("before", raw[:at]), ("behind", raw[end:])):
+        bad = (part != GUARD_BYTE).nonzero()
+        assert bad.numel() == 0, "%d bytes %s the output written, the first %d bytes from its %s" % (
+            bad.numel(), name, at - int(bad[-1]) if name == "before" else int(bad[0]),
+            "start" if name == "before" else "end")
+
+
 def device_generate(lib, g, dist, n, params=(), mis=0):
     """One generate call into device memory placed (mis * itemsize) bytes past a 512-byte
     boundary (the caching allocator's alignment), which matches the host placement of the
-    oracle ((mis * itemsize) mod 64 past a 64-byte boundary) for mis * itemsize < 64;
-    returns (status, numpy values)."""
+    oracle ((mis * itemsize) mod 64 past a 64-byte boundary) for mis * itemsize < 64, between
+    guard bytes that must stay as they were; returns (status, numpy values)."""
     import torch
     suffix, dt, _ = pyorc.DISTS[dist]
-    isz = np.dtype(dt).itemsize
-    buf = torch.empty(n + 64 // isz + 16, dtype=torch_dtype(dist), device="cuda")
-    view = buf[mis:mis + n]
+    raw, view, address = guarded_output(n, torch_dtype(dist), mis)
     fn = getattr(lib, "rocrand_" + suffix)
-    st = fn(g, c_void_p(view.data_ptr()), c_size_t(n), *pyorc.dist_args(dist, params))
+    st = fn(g, c_void_p(address), c_size_t(n), *pyorc.dist_args(dist, params))
     torch.cuda.synchronize()
+    check_guards(raw, view)
     return st, view.cpu().numpy().view(dt)
 
 

@@ -62,11 +62,11 @@ def _run_batch(lib, reqs, plan_mode=None):
     bufs, arr = [], (Request * len(reqs))()
     for k, (t, d, seed, offset, n, mis) in enumerate(reqs):
         dt = gu.torch_dtype(DISTS[d][0])
-        buf = torch.zeros(n + 16, dtype=dt, device="cuda")
-        bufs.append(buf)
+        raw, out, address = gu.guarded_output(n, dt, mis)
+        out.zero_()
+        bufs.append((raw, out))
         p = DISTS[d][1]
-        arr[k] = Request(t, d, seed, offset, p[0] if p else 0.0, p[1] if len(p) > 1 else 0.0,
-                         buf[mis:].data_ptr(), n)
+        arr[k] = Request(t, d, seed, offset, p[0] if p else 0.0, p[1] if len(p) > 1 else 0.0, address, n)
     stream = torch.cuda.current_stream().cuda_stream
     if plan_mode is None:
         assert lib.rocrand_b200_generate_batch(arr, len(reqs), ctypes.c_void_p(stream)) == 0
@@ -75,14 +75,15 @@ def _run_batch(lib, reqs, plan_mode=None):
         assert lib.rocrand_b200_create_batch_plan(ctypes.byref(plan), arr, len(reqs),
                                                   ctypes.c_void_p(stream)) == 0
         for _ in range(2):  # the second execution of a graph plan is a replay
-            for b in bufs:
-                b.zero_()
+            for _, out in bufs:
+                out.zero_()
             assert lib.rocrand_b200_execute_batch_plan(plan, plan_mode, ctypes.c_void_p(stream)) == 0
         assert lib.rocrand_b200_destroy_batch_plan(plan) == 0
     torch.cuda.synchronize()
     out = []
-    for (t, d, seed, offset, n, mis), buf in zip(reqs, bufs):
-        out.append(buf[mis:mis + n].cpu().numpy().view(pyorc.DISTS[DISTS[d][0]][1]))
+    for (t, d, seed, offset, n, mis), (raw, values) in zip(reqs, bufs):
+        gu.check_guards(raw, values)
+        out.append(values.cpu().numpy().view(pyorc.DISTS[DISTS[d][0]][1]))
     return out
 
 
