@@ -17,16 +17,18 @@
 //    neither the reduction nor b needs a second word; sin/cos(m C) from a double-double table
 //    over the whole circle (15 KB, so no quadrant to select either); sin b and cos b - 1 by
 //    short series.
-// Both are IEEE operations only (add, mul, fma, sqrt-free), so host and device builds of
-// this header give identical results; the tables are computed in binary128 at build time
-// (rocrand_b200/data/make_precise_tables.c).
+// Both are IEEE operations only (add, mul, fma), so their host and device builds give identical
+// results; the tables are computed in binary128 at build time
+// (rocrand_b200/data/make_precise_tables.c).  (sqrt_inner below starts from an instruction of the
+// device's own and is another function on the host.)
 // Issue bounds the transforms (an fp64 instruction takes two to three cycles of its scheduler:
 // 2.07 with constant operands, 3.03 with three registers, every other about one): a Philox
 // Box-Muller pair took 269 instructions, 108 of them fp64, with a two-step reduction (k pi/2 in
-// three parts, then j/64), the special cases of log in line and sqrt.rn; now 184 and 76.  Normal
-// fp64, 2^25 values a call on one B200, before -> now: Philox 191 -> 141 us, XORWOW 196 -> 139,
-// LFSR113 223 -> 161, MRG32k3a 234 -> 176, MT19937 263 -> 191, MTGP32 274 -> 232, ThreeFry4x64
-// 249 -> 206.  Misses of correct rounding in 3 10^6: sine 32 -> 27, cosine 23 -> 23, log 0.
+// three parts, then j/64), log's special cases and the rounded square root; now 184 and 76.  Normal
+// fp64, 2^25 values a call on one B200, before -> now (the engines' own changes included): Philox
+// 191 -> 141 us, XORWOW 197 -> 125, LFSR113 224 -> 149, MRG32k3a 235 -> 150, MT19937 266 -> 195,
+// MTGP32 274 -> 236, ThreeFry4x64 249 -> 194.  Misses of correct rounding in 3 10^6: sine 32 -> 27,
+// cosine 23 -> 23, log 0.
 #pragma once
 
 #include "precise_tables.inc"
@@ -193,14 +195,25 @@ RB_PM_HD void sincos(double x, double& s_out, double& c_out)
     c_out              = csh + c_low;
 }
 
-// Square root of t = 0 or 2^-200 <= t <= 2^200, correctly rounded but for near-halfway cases
-// within 2^-100 relative: the hardware's 20-bit reciprocal square root y, one third-order step
-// on t y and y / 2, and Markstein's residual correction.  (sqrt.rn's range check and its out of
-// line path are what this saves: the same number of fp64 operations.)
+// Square root of t = 0 or 2^-200 <= t <= 2^200, within 2^-103 relative before its one rounding,
+// so correctly rounded but where the root is as near as that to a midpoint of two doubles.
+// From an approximation y = (1 + d) / sqrt(t) (the reciprocal square root instruction's, |d| <
+// 2^-19), Goldschmidt's coupled pair (R. E. Goldschmidt, "Applications of division by
+// convergence", MIT 1964) g = t y ~ sqrt(t), h = y / 2 ~ 1 / (2 sqrt(t)):
+//   g h = (1 - 2 e) / 2 gives e = 1/2 - g h in one fma, |e| < 2^-18.9;
+//   sqrt(t) = g (1 - 2 e)^(-1/2) = g (1 + e + 3/2 e^2 + 5/2 e^3 + ..): with q = e (1 + 3/2 e),
+//   g1 = g + g q and h1 = h + h q are 5/2 |e|^3 < 2^-55 and their roundings off, |n| < 2^-52 in
+//   all for g1 = sqrt(t) (1 + n).
+// Then the residual correction by one fma each (P. Markstein, "Computation of elementary functions
+// on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990): r = t - g1^2 = -t (2 n +
+// n^2), and g1 + r h1 = sqrt(t) (1 - n^2 / 2 and less than 2^-52 |n|), rounded once.
+// 2^25 Philox normals fp64 on one B200 with the rounded root's intrinsic -> this: 146 -> 141 us;
+// MT19937 217 -> 193.  On the device the function is not IEEE operations alone (the host has
+// std::sqrt); tests/test_device_math_gpu.py compares the device's with the rounded root.
 RB_PM_HD double sqrt_inner(double t)
 {
 #if defined(__CUDA_ARCH__)
-    // t = 0 seeds with a tiny number instead, and t y = 0 then stays 0
+    // t = 0 starts from a tiny number instead, and t y = 0 then stays 0
     const double seed = __hiloint2double(max(__double2hiint(t), 0x02000000), __double2loint(t));
     double       y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(seed));

@@ -12,10 +12,13 @@ namespace rb200
 // ---- distributions over a Sobol value (sobol_*_distribution, uniform.hpp:351-442,
 //      normal.hpp:272-330, log_normal.hpp:296-370, poisson.hpp CDF method) ----
 
-// sqrt(x) rounded to nearest for x = 0 and 2^-26 <= x < 2^10: the hardware's reciprocal square
-// root y (at most 1e18, so that x = 0 gives 0) and one residual correction (Markstein).  Equal to
-// sqrt.rn on every float of that range (compared exhaustively on the device), without its range
-// check.
+// sqrt(x) rounded to nearest, for x = 0 and 2^-26 <= x < 2^10.  From y = (1 + d) / sqrt(x) (the
+// reciprocal square root instruction's, |d| <= 2^-22.9 as PTX documents it; held at 1e18, so that
+// x = 0 gives 0): g = x y = sqrt(x) (1 + n), |n| < 2^-22, and Markstein's residual correction (IBM
+// J. Res. Dev. 34, 1990), r = x - g^2 = -x (2 n + n^2) in one fma and g + r y / 2 = sqrt(x) (1 -
+// n^2 / 2 and less than 2^-21.5 |n|) in another: within 2^-43 before its one rounding.  A root can
+// be 2^-50 from a midpoint of two floats, so that alone leaves a few in doubt:
+// tests/test_device_math_gpu.py compares all floats of the range with the rounded root.
 RB_HD float sqrt_mid(float x)
 {
 #if defined(__CUDA_ARCH__)
@@ -37,9 +40,9 @@ RB_HD float times2n_plus(float a, float b, float c) { RB_PICK(__fmaf_rn(a, b, c)
 // host C library's logf (logf_replay.cuh), which the outer cancellation amplifies.  The
 // logarithm is -inf only at |x| = 1 (0 results), never NaN; the inner root's argument lies in
 // [18, 2^9), the outer one's is 0 or at least 2^-22 (a difference of floats in [4, 2^5)).
-// Issue bounds the kernel: 139 instructions a point with a float-float logarithm of 2^-44, an
-// integer distance from the midpoint and sqrt.rn; 64 dimensions x 2^20 points of normal fp32 on
-// one B200 305 -> 235 us (scrambled Sobol64 348 -> 246).
+// Issue bounds the kernel: it was 139 instructions a point with a float-float logarithm of 2^-44,
+// an integer distance from the midpoint and the rounded root's intrinsic; 64 dimensions x 2^20
+// points of normal fp32 on one B200 305 -> 235 us (scrambled Sobol64 348 -> 246).
 RB_HD float erfinv_f(float x, const lr::Table& logf_table)
 {
     const float t = ieee::fmul(ieee::fsub(1.0f, x), ieee::fadd(1.0f, x));
