@@ -76,9 +76,9 @@ inline float2 box_muller_host(float u, float a)
 
 // ---- fp32 and half Box-Muller functors: two units at a time ----
 // Such a functor names the uniforms and angles of two units (`uniforms`, `angles`: the inputs'
-// own rounding steps) and its parameters; normal_pair makes both units' outputs.  On the device one unit alone is the same computation with the unit taken twice, so
-// a value does not depend on whether it was made alone or beside another; on the host each
-// unit is made with the C library.
+// own rounding steps) and its parameters; normal_pair makes both units' outputs.  On the device
+// one unit alone is the same computation with the unit taken twice, so a value does not depend on
+// whether it was made alone or beside another; on the host each unit is made with the C library.
 
 // rocrand_uniform.h:61-64 and rocrand_normal.h:51-66 of two 32-bit words.
 RB_HD nm::F2 uniform_pair(uint32_t x0, uint32_t x1)

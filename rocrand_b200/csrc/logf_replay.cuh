@@ -10,17 +10,17 @@
 // formula can produce, 0.93 % of its results are the other neighbour of the exact value.
 //
 // Method.  The kernels evaluate the logarithm L = hi + lo as a pair of floats (base(): a
-// table-driven reduction in single precision; at worst 2^-7.6 of an ulp off, 2^-11 below 0.9) and take f = hi, its rounding to float.  A host result that differs
-// from f can only be f's other neighbour on L's side of f (the host's error is below one ulp),
-// and only where L lies close to the midpoint between the two.  The build
-// (rocrand_b200/data/make_logf_replay.cpp) runs the host's logf over every argument the formula
-// can reach and records
+// table-driven reduction in single precision; at worst 2^-7.6 of an ulp off, 2^-11 below 0.9) and
+// take f = hi, its rounding to float.  A host result that differs from f can only be f's other
+// neighbour on L's side of f (the host's error is below one ulp), and only where L lies close to
+// the midpoint between the two.  The build (rocrand_b200/data/make_logf_replay.cpp) runs the host's
+// logf over every argument the formula can reach and records
 //  * per bucket of arguments (the float's bits >> kBucketShift) and side of f (L below f, L
 //    above f), the smallest |lo| / 2^exponent(hi) of an argument whose host result differs from
 //    f, as the upper 16 bits of a float, rounded down (none: infinity);
 //  * those arguments, as a set: a bucketed two-choice hash table of 32-bit keys, four per
 //    16-byte bucket, so a lookup is two independent 16-byte loads.
-// An argument that reaches its bucket's threshold for its side tests membership (about 1.5 % of
+// An argument that reaches its bucket's threshold for its side tests membership (1.18 % of
 // arguments), and a member returns f's neighbour on L's side; all others return f.  The build
 // then replays every reachable argument through this same code on the host and requires the
 // host's logf result for each, which is also what makes base()'s accuracy enough.  base() and
@@ -137,8 +137,9 @@ RB_PM_HD float threshold_of(uint32_t word, float lo)
 RB_PM_HD uint32_t bucket1(uint32_t key, uint32_t lb) { return (key * kHash1) >> (32 - lb); }
 RB_PM_HD uint32_t bucket2(uint32_t key, uint32_t lb) { return (key * kHash2) >> (32 - lb); }
 
-// The host C library's logf(t) for an argument of the inverse-erf normal, t >= 2^-24 or so (t = 0
-// gives some number).
+// The host C library's logf(t) for an argument that the inverse-erf normal can produce, and for no
+// other (the build replays just those: base() is no more accurate than they need, and a t above 1
+// has no bucket); t = 0 gives some number.
 RB_PM_HD float logf_host(float t, const Table& tb)
 {
     float          lo;

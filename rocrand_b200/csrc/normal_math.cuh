@@ -1,26 +1,31 @@
 // normal_math.cuh -- single-precision Box-Muller on two units at a time.
 //
 // A unit is a uniform u in (0, 1] and an angle a in [0, 2 pi], both floats; its results are
-// sqrt(-2 log u) sin a and sqrt(-2 log u) cos a.  Every floating-point step runs on the two
-// units' values packed in one 64-bit register pair (add / mul / fma .rn.f32x2: one issue slot
-// for two roundings, each rounded as the scalar operation), which is what the normal kernels
-// are short of: the library form (logf, sqrt.rn, sincosf, one unit at a time) ran at 84 % of
-// the issue slots with the FMA pipe 47 % busy.
+// sqrt(-2 log u) sin a and sqrt(-2 log u) cos a.  The floating-point steps run on the two units'
+// values packed in one 64-bit register pair (add / mul / fma .rn.f32x2).  The kernels are short of
+// instructions issued and not of the FMA pipe: with CUDA's logf, square root and sincosf, one unit
+// at a time, they ran at 84 % of the issue slots with that pipe 47 % busy.  (A packed fma holds
+// the pipe for 2.3 cycles with constant operands and 3.1 with three registers, a scalar one for 1.)
+// A product and a sum are each rounded only where nothing joins them: a packed mul whose result
+// goes into a packed add has come out rounded once, as an fma.  Where two roundings are needed the
+// products are scalar (angle_pair in dist.cuh); here every sum of a product is an fma to begin with.
 //  * u = 2^k z with z in [2/3, 4/3): m = 2 log u = g + g^2 Q(g) + k 2 ln 2 with g = 2z - 2
 //    exact and Q a degree-8 minimax polynomial (2^-28 relative; relative to the whole
 //    logarithm where k != 0);
 //  * the radius with a minus sign (which saves the residual's negation) by one residual step
-//    on the hardware reciprocal square root y = (-m)^-1/2 (Markstein's correction: s0 = m y,
-//    s = s0 + (s0^2 + m) y / 2), 0 for m = 0;
+//    on the hardware reciprocal square root y = (-m)^-1/2 (P. Markstein, IBM J. Res. Dev. 34,
+//    1990: s0 = m y, s = s0 + (s0^2 + m) y / 2), 0 for m = 0;
 //  * a = n pi/2 + r, n by the rounding of a 2/pi, pi/2 in three parts of which the first
 //    product is exact; sin r and cos r by minimax polynomials on |r| <= pi/4 (2^-28, 2^-33);
 //  * n swaps the two, and its signs and the radius' minus go into the radius.
 // The coefficients are derived by rocrand_b200/data/make_fp32_polynomials.py.  Measured
 // on the device against 64 bits from the same uniforms, the products are 4.52e-8 off (2-norm),
-// those of the library form 4.72e-8; logarithm 0.87 ulp at most, sine and cosine 1.5.
-// Normal fp32, 2^26 values a call on one B200, library form -> this: Philox 125 -> 94 us,
-// XORWOW 122 -> 86, MRG32k3a 234 -> 188, MT19937 190 -> 142, ThreeFry4x32 168 -> 150,
-// ThreeFry2x64 206 -> 176, MTGP32 202 -> 165, LFSR113 156 -> 118; half within 2 % of the same.
+// those of the library form 4.72e-8; logarithm 0.87 ulp at most, sine and cosine 1.5
+// (tests/test_device_math_gpu.py and, for the host's build, tests/test_normal_math.py hold it there).
+// Normal fp32, 2^26 values a call on one B200, library form -> now (the engines' own changes
+// included): Philox 124 -> 94 us, XORWOW 123 -> 77, MRG32k3a 233 -> 149, MT19937 191 -> 136,
+// ThreeFry4x32 167 -> 137, ThreeFry2x64 206 -> 169, MTGP32 202 -> 151, LFSR113 156 -> 104; half
+// 108 -> 80, 120 -> 75, 177 -> 111, 170 -> 109, 130 -> 101, 214 -> 175, 185 -> 114, 138 -> 89.
 #pragma once
 
 #include "ieee.cuh"
