@@ -93,14 +93,6 @@ RB_PM_HD double from_bits(uint64_t u)
     return x;
 }
 
-// s + e == a + b exactly
-RB_PM_HD void two_sum(double a, double b, double& s, double& e)
-{
-    s              = a + b;
-    const double bb = s - a;
-    e              = (a - (s - bb)) + (b - bb);
-}
-
 // s + e == a + b exactly when a == 0 or |a| >= |b| (Dekker's fast two-sum)
 RB_PM_HD void fast_two_sum(double a, double b, double& s, double& e)
 {
@@ -228,12 +220,6 @@ RB_PM_HD double sqrt_inner(double t)
 #else
     return std::sqrt(t);
 #endif
-}
-
-// Natural logarithm of a float, correctly rounded except in rare double-rounding cases.
-RB_PM_HD float logf(float x)
-{
-    return static_cast<float>(log(static_cast<double>(x)));
 }
 
 } // namespace pm

@@ -23,7 +23,7 @@ int main(int argc, char** argv)
     const long      n = argc > 1 ? std::atol(argv[1]) : 200000;
     std::mt19937_64 rng(42);
     double          max_log = 0, max_sin = 0, max_cos = 0, max_glog = 0, max_gsin = 0, max_gcos = 0;
-    long            miss_log = 0, miss_sin = 0, miss_cos = 0, miss_logf = 0, miss_glog = 0, miss_gsin = 0;
+    long            miss_log = 0, miss_sin = 0, miss_cos = 0, miss_glog = 0, miss_gsin = 0;
     for(long t = 0; t < n; t++)
     {
         // log: the Box-Muller inputs (k + 1) 2^-53 and general normal numbers
@@ -37,9 +37,6 @@ int main(int argc, char** argv)
         max_glog           = std::fmax(max_glog, std::fabs(ulp_err(g, lx)));
         miss_log += a != static_cast<double>(lx);
         miss_glog += g != static_cast<double>(lx);
-        const float xf = static_cast<float>(x);
-        if(xf > 0.0f)
-            miss_logf += rb200::pm::logf(xf) != static_cast<float>(logq((__float128)xf));
         // sin/cos on (0, 2 pi]: the Box-Muller angles w * pi, w = k 2^-52
         const double ang = (static_cast<double>(rng() >> 11) + 1.0) * 0x1p-52 * 3.141592653589793;
         double       s, c;
@@ -83,7 +80,6 @@ int main(int argc, char** argv)
     std::printf("log_near %.6f %ld %ld\n", max_near, miss_near, n_near);
     std::printf("sin %.6f %ld %ld\n", max_sin, miss_sin, n);
     std::printf("cos %.6f %ld %ld\n", max_cos, miss_cos, n);
-    std::printf("logf 0 %ld %ld\n", miss_logf, n);
     std::printf("glibc_log %.6f %ld %ld\n", max_glog, miss_glog, n);
     std::printf("glibc_sin %.6f %ld %ld\n", max_gsin, miss_gsin, n);
     // special values
