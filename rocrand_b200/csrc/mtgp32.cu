@@ -21,6 +21,7 @@
 #include "generators.hpp"
 #include "host_exec.hpp"
 #include "launch.cuh"
+#include "mtgp32_params.hpp"
 #include "stateful_engines.cuh"
 
 #include <cuda_runtime.h>
@@ -38,12 +39,8 @@ namespace rb200
 namespace
 {
 
-constexpr int      kMtgpN     = 351;
 constexpr int      kMtgpState = 1024;
 constexpr int      kMtgpMask  = 1023;
-constexpr uint32_t kMtgpGens  = 512;
-constexpr uint32_t kMtgpBlock = 256;
-constexpr int      kMtgpWords = 36; // pos, sh1, sh2, tbl[16], tmp_tbl[16], mask
 
 struct MtgpArgs
 {
@@ -64,9 +61,7 @@ constexpr unsigned kMtgpUnits = F::iw == 1 ? 4u : F::iw == 2 ? 2u : 4u;
 
 // Words after the ring that repeat its first ones: a step reads up to pos + 255 words ahead of
 // its offset, pos <= kMtgpReach, the last of the four offsets being 768.
-constexpr int kMtgpReach  = 95;
-constexpr int kMtgpMirror = 96;
-static_assert(kMtgpBlock + kMtgpReach <= kMtgpN, "a step reads no word that it writes");
+constexpr int kMtgpMirror = kMtgpReach + 1;
 
 // The ring in shared memory starts at the call's offset, so that the four block steps of a turn
 // work at the constant offsets 0, 256, 512 and 768 and every address is the thread's base plus
@@ -313,7 +308,7 @@ void mtgp_fill_host(const MtgpArgs& a, const F& f)
 }
 
 // Parameter sets on each device, uploaded once.
-const uint32_t* device_params()
+const uint32_t* device_params(const uint32_t* host_params)
 {
     static std::mutex                   mu;
     static std::vector<const uint32_t*> ptr(64, nullptr);
@@ -321,14 +316,11 @@ const uint32_t* device_params()
     std::lock_guard<std::mutex>         lock(mu);
     if(ptr[dev])
         return ptr[dev];
-    const size_t bytes = static_cast<size_t>(rb200_mtgp32_params_end - rb200_mtgp32_params_begin);
-    const size_t want  = 12 + sizeof(uint32_t) * kMtgpWords * kMtgpGens;
-    if(bytes != want || std::memcmp(rb200_mtgp32_params_begin, "RBMTGP01", 8) != 0)
+    constexpr size_t bytes = sizeof(uint32_t) * kMtgpWords * kMtgpGens;
+    void*            d     = nullptr;
+    if(cudaMalloc(&d, bytes) != cudaSuccess)
         return nullptr;
-    void* d = nullptr;
-    if(cudaMalloc(&d, want - 12) != cudaSuccess)
-        return nullptr;
-    if(cudaMemcpy(d, rb200_mtgp32_params_begin + 12, want - 12, cudaMemcpyHostToDevice) != cudaSuccess)
+    if(cudaMemcpy(d, host_params, bytes, cudaMemcpyHostToDevice) != cudaSuccess)
     {
         cudaFree(d);
         return nullptr;
@@ -381,12 +373,11 @@ public:
         // that a generate call recorded by a stream capture allocates nothing
         if(m_poisson.reserve() != ROCRAND_STATUS_SUCCESS)
             return ROCRAND_STATUS_ALLOCATION_FAILED;
-        const size_t pbytes = static_cast<size_t>(rb200_mtgp32_params_end - rb200_mtgp32_params_begin);
-        if(pbytes != 12 + sizeof(uint32_t) * kMtgpWords * kMtgpGens
-           || std::memcmp(rb200_mtgp32_params_begin, "RBMTGP01", 8) != 0)
+        const uint32_t* const host_params = mtgp_parameter_sets(
+            rb200_mtgp32_params_begin, static_cast<size_t>(rb200_mtgp32_params_end - rb200_mtgp32_params_begin));
+        if(host_params == nullptr)
             return ROCRAND_STATUS_INTERNAL_ERROR;
-        m_params = m_host_exec ? reinterpret_cast<const uint32_t*>(rb200_mtgp32_params_begin + 12)
-                               : device_params();
+        m_params = m_host_exec ? host_params : device_params(host_params);
         if(m_params == nullptr)
             return ROCRAND_STATUS_ALLOCATION_FAILED;
         constexpr size_t kRingWords = static_cast<size_t>(kMtgpGens) * kMtgpState;
@@ -400,7 +391,6 @@ public:
             }
         }
         // rocrand_make_state_mtgp32 / rocrand_mtgp32_init_state on the host (2 MiB)
-        const auto*              host_params = reinterpret_cast<const uint32_t*>(rb200_mtgp32_params_begin + 12);
         std::vector<uint32_t>    rings(kRingWords, 0u);
         const unsigned long long seed = m_seed ^ (m_seed >> 32);
         for(uint32_t i = 0; i < kMtgpGens; i++)
